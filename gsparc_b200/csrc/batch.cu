@@ -304,7 +304,9 @@ __global__ void k_brows(const uint64_t *__restrict__ xkeys, int kbx, const BPrep
 // (their output count is their product count), other rows with more than the job's light limit of products are
 // heavy, the rest with products are light.  Rows outside [range[0],
 // range[1]) (a shard) get no class and no output.
-__global__ void k_bclass(const uint64_t *__restrict__ row_prod, const uint32_t *__restrict__ row_runs,
+// Also lists the matched X nonzeros (mrun), the runs of every row in order.
+__global__ void k_bclass(const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ mpre,
+                         uint32_t *__restrict__ mrun, const uint64_t *__restrict__ row_prod, const uint32_t *__restrict__ row_runs,
                          const uint16_t *__restrict__ row_job, const BPrep *__restrict__ jobs,
                          const unsigned int *__restrict__ ydup,
                          const uint64_t *__restrict__ nrows_dev, const uint64_t *__restrict__ range, uint64_t nx,
@@ -314,6 +316,7 @@ __global__ void k_bclass(const uint64_t *__restrict__ row_prod, const uint32_t *
     const uint64_t r0 = range ? range[0] : 0, r1 = range ? range[1] : nr;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nx; r += stride) {
+        if (cnt[r]) mrun[mpre[r]] = (uint32_t)r;  // r as a nonzero
         uint8_t h = 0, l = 0, st = 0;
         uint64_t p = 0;
         if (r < nr && r >= r0 && r < r1) {
@@ -631,7 +634,7 @@ struct GroupPlan {
     DBuf<float> xperm, yperm, xvals, yvals;
     DBuf<uint64_t> ykeys;  // sorted Y keys (the single-run-row copy reads y_f from them)
     DBuf<BatchJob> d_acc;
-    DBuf<uint32_t> rank, pos, cnt, row_start, units, H, H2, SR, row_xi, cursor, pend;
+    DBuf<uint32_t> rank, pos, cnt, mpre, mrun, row_start, units, H, H2, SR, row_xi, cursor, pend;
     DBuf<uint64_t> cols, xprefix, row_xf, sprefix, row_off;
     DBuf<uint16_t> row_job;
     DBuf<uint32_t> Hc;         // heavy rows grouped by chunk (several chunks only)
@@ -695,9 +698,9 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         max_light = std::max(max_light, j->light_max);
     }
     // light units hold rows whose first product falls in one bin of light_bin
-    // products: fewer than light_bin + light_max <= kLightCap products
-    const uint64_t light_bin = std::max<uint64_t>(
-        1, std::min<uint64_t>(kLightUnitMax - kLightRowMax, (uint64_t)kLightCap - std::min<uint64_t>(max_light, kLightCap - 1)));
+    // products: fewer than light_bin + light_max <= light_cap products
+    const uint64_t light_cap = max_light <= kLightRowMax ? kLightCap / 2 : kLightCap;
+    const uint64_t light_bin = light_cap - std::min<uint64_t>(max_light, light_cap - 1);
     GS_REQUIRE(kbx + jb <= 64 && kby + jb <= 64, GSPARC_EINTERNAL, "batch group keys wider than 64 bits");
 
     cudaEvent_t *ev = ctx->ev;
@@ -836,7 +839,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     DBuf<uint16_t> row_job(A, nxb, s);
     DBuf<uint32_t> H(A, nxb, s), hc(A, nx + 1, s), units(A, 2 * nxb, s);
     DBuf<uint64_t> lpre(A, nx + 1, s);
-    DBuf<uint32_t> mpre(A, nx + 1, s), row_runs(A, nxb, s), row_xi(A, nxb, s), SR(A, nxb, s);
+    DBuf<uint32_t> mpre(A, nx + 1, s), row_runs(A, nxb, s), row_xi(A, nxb, s), SR(A, nxb, s), mrun(A, nxb, s);
     DBuf<uint64_t> sprefix(A, nx + 1, s);
     DBuf<uint32_t> row_nnz(A, nxb, s);
     GS_CUDA(cudaMemsetAsync(row_nnz.get(), 0, 4 * nxb, s));
@@ -885,7 +888,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
             range = cnts.get() + 9;
         }
         if (nx) {
-            k_bclass<<<grid_for(nx), kThreads, 0, s>>>(row_prod, row_runs, row_job, d_bp, d_ydup, cnts.get() + 2,
+            k_bclass<<<grid_for(nx), kThreads, 0, s>>>(cnt, mpre, mrun, row_prod, row_runs, row_job, d_bp, d_ydup, cnts.get() + 2,
                                                         range, nx, heavy, lnz, sflag, brk, lp, row_nnz);
             count_launch();
             GS_CUDA(cudaGetLastError());
@@ -981,6 +984,9 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     aa.pos = pos;
     aa.cnt = cnt;
     aa.xprefix = xprefix;
+    aa.mpre = mpre;
+    aa.mrun = mrun;
+    aa.light_cap = (uint32_t)light_cap;
     aa.xval = xvals;
     aa.yrank = rank;
     aa.yval = yvals;
@@ -1185,6 +1191,8 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         keep->rank = std::move(rank);
         keep->pos = std::move(pos);
         keep->cnt = std::move(cnt);
+        keep->mpre = std::move(mpre);
+        keep->mrun = std::move(mrun);
         keep->row_start = std::move(row_start);
         keep->units = std::move(units);
         keep->H = std::move(H);

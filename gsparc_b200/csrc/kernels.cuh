@@ -82,6 +82,8 @@ struct AccArgs {
     const uint32_t *pos;
     const uint32_t *cnt;
     const uint64_t *xprefix;
+    const uint32_t *mpre;      // [nx + 1] matched X nonzeros before each one
+    const uint32_t *mrun;      // [matched] the matched X nonzeros, ascending
     const float *xval;
     // Y side
     const uint32_t *yrank;
@@ -96,6 +98,7 @@ struct AccArgs {
     // work
     const uint32_t *units;     // light: pairs (r0, r1); heavy and stream: row ids
     uint32_t nunits;
+    uint32_t light_cap;        // light: products of a unit stay below this (at most kLightCap)
     unsigned int *work_counter;
     uint32_t *cursor;          // [nx] scratch (heavy path): next unprocessed Y entry per run
     uint32_t *pend;            // [nx] scratch (heavy path): end of the run's part in the window
@@ -125,10 +128,8 @@ constexpr int kHeavyCap = 8192;    // output slots (compensated accumulators) pe
                                    // (sized so two CTAs fit one SM's shared memory)
 constexpr int kHeavyMaxRuns = 512;   // runs flattened per batch
 constexpr int kGallopWarpRuns = 64;  // up to this many runs per batch: one warp per run search
-constexpr int kLightCap = 4096;    // on-chip ESC capacity (products per unit)
-constexpr int kLightThreads = 512;
+constexpr int kLightCap = 4096;    // on-chip ESC capacity (products per unit); half of it for rows of up to kLightRowMax
 constexpr uint64_t kLightRowMax = 1024;   // rows with at most this many products are light
-constexpr uint64_t kLightUnitMax = 3072;  // products per light unit
 
 // Output-key width and column table of the job that owns `row`.
 __device__ __forceinline__ void row_job_params(const AccArgs &a, uint32_t row, int &y_nfbits,
