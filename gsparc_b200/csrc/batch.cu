@@ -16,7 +16,7 @@
 // symbolic and ONE numeric persistent launch take the units of all jobs from
 // one work counter.  Unit planning (light units, heavy rows) runs on the
 // device, so a group needs two host round trips before its numeric launch
-// whatever its number of jobs.  Each job's output is the contiguous range of
+// whatever its number of jobs (the planning kernels are in rows.cu).  Each job's output is the contiguous range of
 // the group's sorted output that belongs to it, delivered to the job's sink.
 #include <cub/cub.cuh>
 
@@ -27,6 +27,7 @@
 
 #include "engine.h"
 #include "kernels.cuh"
+#include "rows.h"
 #include "verify.h"
 #include "wide.h"
 
@@ -67,13 +68,6 @@ struct BLin {
     const uint64_t *idx;  // SoA idx[m * nnz + k]
     const float *val;
     uint64_t nnz;
-};
-
-// Per-job constants of the batched prep kernels.
-struct BPrep {
-    int x_ncbits;
-    int y_nfbits;
-    uint64_t light_max;  // rows with more products go to the windowed accumulator
 };
 
 // Per-job summary after the symbolic pass (entry g holds the totals).
@@ -141,31 +135,6 @@ __global__ void k_bvals(const BLin *__restrict__ tab, const uint64_t *__restrict
     }
 }
 
-// Y: run boundaries of (job, contract key) and the prefixed free index.
-// A job whose Y repeats a coordinate gets ydup[job] set: its runs may hold a
-// free index twice, so none of its rows is streamed.
-__global__ void k_by_split(const uint64_t *__restrict__ ykeys, uint64_t ny, int kby,
-                           const BPrep *__restrict__ jobs, uint8_t *__restrict__ run_flag,
-                           uint64_t *__restrict__ yfk, unsigned int *__restrict__ ydup) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t km = low_mask(kby);
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ny; i += stride) {
-        const uint64_t key = ykeys[i];
-        const uint64_t j = shr(key, kby);
-        const int nfb = jobs[j].y_nfbits;
-        const uint64_t loc = key & km;
-        const uint64_t c = shr(loc, nfb);
-        uint8_t flag = 1;
-        if (i > 0) {
-            const uint64_t pk = ykeys[i - 1];
-            flag = (shr(pk, kby) != j) || (shr(pk & km, nfb) != c);
-            if (pk == key) atomicOr(&ydup[j], 1u);
-        }
-        run_flag[i] = flag;
-        yfk[i] = shl(j, kby) | (loc & low_mask(nfb));
-    }
-}
-
 // Distinct prefixed free indices -> plain free indices (the column tables).
 __global__ void k_bcols(const uint64_t *__restrict__ uniq, const uint64_t *__restrict__ ncols_dev,
                         int kby, uint64_t *__restrict__ cols) {
@@ -207,23 +176,6 @@ __global__ void k_brank(const uint64_t *__restrict__ ykeys, uint64_t ny, int kby
     }
 }
 
-__global__ void k_bruns(const uint64_t *__restrict__ ykeys, int kby, const BPrep *__restrict__ jobs,
-                        const uint32_t *__restrict__ rs, const uint64_t *__restrict__ nruns_dev,
-                        uint64_t ny, uint64_t *__restrict__ run_key, uint32_t *__restrict__ run_start_out) {
-    const uint64_t nr = *nruns_dev;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t km = low_mask(kby);
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= nr; r += stride) {
-        if (r < nr) {
-            const uint64_t key = ykeys[rs[r]];
-            const uint64_t j = shr(key, kby);
-            run_key[r] = shl(j, kby) | shr(key & km, jobs[j].y_nfbits);
-        } else {
-            run_start_out[nr] = (uint32_t)ny;
-        }
-    }
-}
-
 // reference: include/gsparc/indexMatch.cuh:67-118, over the run table of all
 // jobs: the search key is (job, contract key).
 __global__ void k_bmatch(const uint64_t *__restrict__ xkeys, uint64_t nx, int kbx, int kby,
@@ -257,97 +209,21 @@ __global__ void k_bmatch(const uint64_t *__restrict__ xkeys, uint64_t nx, int kb
     }
 }
 
-// Row table: first X nonzero, free index, job and matched products of every
-// row, the number of its X nonzeros that match (runs) and, for rows with one
-// run, which nonzero that is.
-__global__ void k_brows(const uint64_t *__restrict__ xkeys, int kbx, const BPrep *__restrict__ jobs,
-                        const uint32_t *__restrict__ rs, const uint64_t *__restrict__ nrows_dev,
-                        uint64_t nx, const uint64_t *__restrict__ xprefix, const uint32_t *__restrict__ mpre,
-                        uint32_t *__restrict__ row_start, uint64_t *__restrict__ row_xf,
-                        uint16_t *__restrict__ row_job, uint64_t *__restrict__ row_prod,
-                        uint32_t *__restrict__ row_runs, uint32_t *__restrict__ row_xi) {
-    const uint64_t nr = *nrows_dev;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t km = low_mask(kbx);
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= nr; r += stride) {
-        if (r == nr) {
-            row_start[nr] = (uint32_t)nx;
-            continue;
-        }
-        const uint32_t a = rs[r];
-        const uint32_t b = (r + 1 < nr) ? rs[r + 1] : (uint32_t)nx;
-        const uint64_t key = xkeys[a];
-        const uint64_t j = shr(key, kbx);
-        row_start[r] = a;
-        row_xf[r] = shr(key & km, jobs[j].x_ncbits);
-        row_job[r] = (uint16_t)j;
-        row_prod[r] = xprefix[b] - xprefix[a];
-        const uint32_t runs = mpre[b] - mpre[a];
-        row_runs[r] = runs;
-        if (runs == 1) {
-            // the nonzero i in [a, b) with mpre[i] == mpre[a] < mpre[i + 1]
-            uint32_t lo = a, hi = b;  // first i in (a, b] with mpre[i] > mpre[a], minus one
-            const uint32_t m0 = mpre[a];
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (mpre[mid + 1] <= m0)
-                    lo = mid + 1;
-                else
-                    hi = mid;
-            }
-            row_xi[r] = lo;
-        }
-    }
-}
-
-// Row classes: single-run rows of jobs without repeated Y coordinates stream
-// (their output count is their product count), other rows with more than the job's light limit of products are
-// heavy, the rest with products are light.  Rows outside [range[0],
-// range[1]) (a shard) get no class and no output.
-// Also lists the matched X nonzeros (mrun), the runs of every row in order.
-__global__ void k_bclass(const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ mpre,
-                         uint32_t *__restrict__ mrun, const uint64_t *__restrict__ row_prod, const uint32_t *__restrict__ row_runs,
-                         const uint16_t *__restrict__ row_job, const BPrep *__restrict__ jobs,
-                         const unsigned int *__restrict__ ydup,
-                         const uint64_t *__restrict__ nrows_dev, const uint64_t *__restrict__ range, uint64_t nx,
-                         uint8_t *__restrict__ heavy, uint8_t *__restrict__ lnz, uint8_t *__restrict__ sflag,
-                         uint8_t *__restrict__ brk, uint64_t *__restrict__ lp, uint32_t *__restrict__ row_nnz) {
-    const uint64_t nr = *nrows_dev;
-    const uint64_t r0 = range ? range[0] : 0, r1 = range ? range[1] : nr;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < nx; r += stride) {
-        if (cnt[r]) mrun[mpre[r]] = (uint32_t)r;  // r as a nonzero
-        uint8_t h = 0, l = 0, st = 0;
-        uint64_t p = 0;
-        if (r < nr && r >= r0 && r < r1) {
-            p = row_prod[r];
-            const uint16_t j = row_job[r];
-            st = row_runs[r] == 1 && !ydup[j];
-            h = !st && p > jobs[j].light_max;
-            l = !st && !h && p > 0;
-            if (st) row_nnz[r] = (uint32_t)p;
-        }
-        heavy[r] = h;
-        lnz[r] = l;
-        sflag[r] = st;
-        brk[r] = h | st;
-        lp[r] = l ? p : 0;
-    }
-}
-
 // Row range of one shard of a single job: shard s starts at the first row
 // whose product midpoint reaches s/n of the job's products, i.e. the first r
-// with n * (P[r] + P[r+1]) >= 2 * s * P[nrows] (P = row product prefix), the
-// exact-integer form of the host planner gs::plan_shards.
+// with n * (P[r] + P[r+1]) >= 2 * s * P[nrows] (P = row product prefix: the
+// products before the row's first nonzero), the exact-integer form of the host
+// planner gs::plan_shards.
 // range = {first row, end row, products of the shard}.
-__device__ uint64_t shard_bound(const uint64_t *P, uint64_t nr, int s, int n) {
+__device__ uint64_t shard_bound(const uint64_t *xprefix, const uint32_t *row_start, uint64_t nr, int s, int n) {
     if (s <= 0) return 0;
     if (s >= n) return nr;
-    const unsigned __int128 target = (unsigned __int128)2 * (unsigned)s * P[nr];
+    const unsigned __int128 target = (unsigned __int128)2 * (unsigned)s * xprefix[row_start[nr]];
     uint64_t lo = 0, hi = nr;
     while (lo < hi) {
         const uint64_t mid = (lo + hi) >> 1;
-        if ((unsigned __int128)(unsigned)n * ((unsigned __int128)P[mid] + P[mid + 1]) >= target)
+        if ((unsigned __int128)(unsigned)n *
+                ((unsigned __int128)xprefix[row_start[mid]] + xprefix[row_start[mid + 1]]) >= target)
             hi = mid;
         else
             lo = mid + 1;
@@ -355,84 +231,30 @@ __device__ uint64_t shard_bound(const uint64_t *P, uint64_t nr, int s, int n) {
     return lo;
 }
 
-__global__ void k_shard_range(const uint64_t *__restrict__ P, const uint64_t *__restrict__ nrows_dev, int shard,
-                              int nshards, uint64_t *__restrict__ range) {
+__global__ void k_shard_range(const uint64_t *__restrict__ xprefix, const uint32_t *__restrict__ row_start,
+                              const uint64_t *__restrict__ nrows_dev, int shard, int nshards,
+                              uint64_t *__restrict__ range, const unsigned int *__restrict__ err) {
+    if (*err & kScanErr) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         const uint64_t nr = *nrows_dev;
-        const uint64_t a = shard_bound(P, nr, shard, nshards), b = shard_bound(P, nr, shard + 1, nshards);
+        const uint64_t a = shard_bound(xprefix, row_start, nr, shard, nshards);
+        const uint64_t b = shard_bound(xprefix, row_start, nr, shard + 1, nshards);
         range[0] = a;
         range[1] = b;
-        range[2] = P[b] - P[a];
+        range[2] = xprefix[row_start[b]] - xprefix[row_start[a]];
     }
 }
 
-__global__ void k_sprod(const uint32_t *__restrict__ SR, const uint64_t *__restrict__ ns_dev, uint64_t nx,
-                        const uint64_t *__restrict__ row_prod, uint64_t *__restrict__ sprod) {
-    const uint64_t ns = *ns_dev;
+// Sort key of the largest-first order of the heavy rows: the product count's
+// binary exponent and two mantissa bits, one 8-bit radix pass (the order only
+// balances the CTAs: a row within a fifth of the next is as good).
+__global__ void k_heavy_sizes(const uint32_t *__restrict__ H, uint64_t nh, const uint64_t *__restrict__ row_prod,
+                              uint8_t *__restrict__ hp) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nx; k += stride)
-        sprod[k] = k < ns ? row_prod[SR[k]] : 0;
-}
-
-// A light unit is a maximal run of light rows with products whose first
-// product falls in the same bin of `bin` products, with no heavy row between
-// them (so it is a contiguous row range): its products stay below
-// bin + light_max.
-__global__ void k_bstart(const uint32_t *__restrict__ L, const uint64_t *__restrict__ nl_dev,
-                         const uint64_t *__restrict__ lpre, const uint32_t *__restrict__ hc,
-                         uint64_t bin, uint64_t nx, uint8_t *__restrict__ sf) {
-    const uint64_t n = *nl_dev;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nx; k += stride) {
-        uint8_t s = 0;
-        if (k < n) {
-            const uint32_t r = L[k];
-            s = 1;
-            if (k > 0) {
-                const uint32_t q = L[k - 1];
-                s = (hc[q] != hc[r]) || (lpre[q] / bin != lpre[r] / bin);
-            }
-        }
-        sf[k] = s;
-    }
-}
-
-// A light unit ends at the next unit start or at the next row of another
-// class (heavy or stream: the breakers B, bc = breakers before each row).
-__global__ void k_bunits(const uint32_t *__restrict__ L, const uint32_t *__restrict__ S,
-                         const uint64_t *__restrict__ cnts, const uint32_t *__restrict__ H,
-                         const uint32_t *__restrict__ hc, uint32_t *__restrict__ units) {
-    const uint64_t nrows = cnts[2], nh = cnts[8], nu = cnts[5];
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < nu; u += stride) {
-        const uint32_t r0 = L[S[u]];
-        const uint64_t next = (u + 1 < nu) ? L[S[u + 1]] : nrows;
-        const uint32_t h = hc[r0];
-        const uint64_t nhv = h < nh ? H[h] : nrows;
-        units[2 * u] = r0;
-        units[2 * u + 1] = (uint32_t)(next < nhv ? next : nhv);
-    }
-}
-
-__global__ void k_gather_prod(const uint32_t *__restrict__ H, uint64_t nh,
-                              const uint64_t *__restrict__ row_prod, uint64_t *__restrict__ hp) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nh; k += stride)
-        hp[k] = row_prod[H[k]];
-}
-
-__global__ void k_bjobout(const uint16_t *__restrict__ row_job, uint64_t nrows,
-                          const uint64_t *__restrict__ row_off, const uint64_t *__restrict__ xprefix,
-                          const uint32_t *__restrict__ hc, const uint64_t *__restrict__ xoffs, int g,
-                          JobOut *__restrict__ out) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j <= g; j += gridDim.x * blockDim.x) {
-        const uint64_t r0 = (j == g) ? nrows : lower_bound_dev<uint16_t>(row_job, 0, nrows, (uint16_t)j);
-        JobOut o;
-        o.row0 = r0;
-        o.out_off = row_off[r0];
-        o.ir_off = xprefix[xoffs[j]];
-        o.heavy0 = hc[r0];
-        out[j] = o;
+    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nh; k += stride) {
+        const uint64_t p = row_prod[H[k]] | 4u;
+        const int e = 63 - __clzll((long long)p);
+        hp[k] = (uint8_t)((e << 2) | ((p >> (e - 2)) & 3u));
     }
 }
 
@@ -476,8 +298,20 @@ struct UnitLists {
     }
 };
 
-// Largest output of one unit.
-__global__ void k_unit_max(UnitLists u, const uint64_t *__restrict__ row_off, uint64_t *__restrict__ out) {
+// Per-job summaries and the largest output of one unit.
+__global__ void k_after_counts(UnitLists u, const uint64_t *__restrict__ row_off, const uint16_t *__restrict__ row_job,
+                               uint64_t nrows, const uint64_t *__restrict__ xprefix,
+                               const uint64_t *__restrict__ xoffs, int g, JobOut *__restrict__ jobs,
+                               uint64_t *__restrict__ out) {
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j <= g; j += gridDim.x * blockDim.x) {
+        const uint64_t r0 = (j == g) ? nrows : lower_bound_dev<uint16_t>(row_job, 0, nrows, (uint16_t)j);
+        JobOut o;
+        o.row0 = r0;
+        o.out_off = row_off[r0];
+        o.ir_off = xprefix[xoffs[j]];
+        o.heavy0 = lower_bound_dev<uint32_t>(u.H, 0, u.nh, (uint32_t)r0);
+        jobs[j] = o;
+    }
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     uint64_t m = 0;
     for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < u.size(); k += stride) {
@@ -550,16 +384,6 @@ __global__ void k_heavy_chunk_keys(const uint32_t *__restrict__ Hs, uint64_t nh,
     }
 }
 
-struct CastU32 {
-    __host__ __device__ uint32_t operator()(uint8_t v) const { return v; }
-};
-struct CastU64 {
-    __host__ __device__ uint64_t operator()(uint32_t v) const { return v; }
-};
-struct NonZero {
-    __host__ __device__ uint32_t operator()(uint32_t v) const { return v != 0; }
-};
-
 template <class T>
 void h2d(T *d, const T *h, size_t n, cudaStream_t s) {
     if (n) GS_CUDA(cudaMemcpyAsync(d, h, sizeof(T) * n, cudaMemcpyHostToDevice, s));
@@ -567,30 +391,6 @@ void h2d(T *d, const T *h, size_t n, cudaStream_t s) {
 template <class T>
 void d2h(T *h, const T *d, size_t n, cudaStream_t s) {
     if (n) GS_CUDA(cudaMemcpyAsync(h, d, sizeof(T) * n, cudaMemcpyDeviceToHost, s));
-}
-
-// Indices i < n with flag[i] != 0, ascending; the count goes to *count (device).
-void select_idx(Arena &A, const uint8_t *flag, uint64_t n, uint32_t *out, uint64_t *count, cudaStream_t s) {
-    if (n == 0) {
-        GS_CUDA(cudaMemsetAsync(count, 0, 8, s));
-        return;
-    }
-    cub::CountingInputIterator<uint32_t> it(0);
-    size_t tmp = 0;
-    GS_CUDA(cub::DeviceSelect::Flagged(nullptr, tmp, it, flag, out, count, (int)n, s));
-    DBuf<uint8_t> t(A, tmp, s);
-    GS_CUDA(cub::DeviceSelect::Flagged(t.get(), tmp, it, flag, out, count, (int)n, s));
-}
-
-// out[0] = 0, out[i+1] = in[0] + ... + in[i] (n + 1 entries).
-template <class It, class T>
-void prefix_sum(Arena &A, It in, T *out, uint64_t n, cudaStream_t s) {
-    GS_CUDA(cudaMemsetAsync(out, 0, sizeof(T), s));
-    if (n == 0) return;
-    size_t tmp = 0;
-    GS_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tmp, in, out + 1, (int)n, s));
-    DBuf<uint8_t> t(A, tmp, s);
-    GS_CUDA(cub::DeviceScan::InclusiveSum(t.get(), tmp, in, out + 1, (int)n, s));
 }
 
 inline int ceil_log2(uint64_t n) {
@@ -638,7 +438,7 @@ struct GroupPlan {
     DBuf<uint64_t> cols, xprefix, row_xf, sprefix, row_off;
     DBuf<uint16_t> row_job;
     DBuf<uint32_t> Hc;         // heavy rows grouped by chunk (several chunks only)
-    DBuf<uint32_t> hbm, row_rb;  // heavy rows' kept column bitmaps (may be empty)
+    DBuf<uint32_t> hbm, row_rb, row_bmw;  // heavy rows' kept column bitmaps (may be empty)
     DBuf<uint64_t> row_bmoff;
     DBuf<unsigned int> flags;  // error bits, work counter, windows swept, spare
     struct Chunk {
@@ -716,6 +516,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     std::vector<uint64_t> xoffs(g + 1, 0), yoffs(g + 1, 0);
     std::vector<BLin> lx(g), ly(g);
     std::vector<BPrep> bp(g);
+    uint64_t col_words = 0;
     for (int j = 0; j < g; ++j) {
         const gsparc_job &J = *G[j]->job;
         const gsparc_tensor *tx = G[j]->tx, *ty = G[j]->ty;
@@ -723,25 +524,43 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         yoffs[j + 1] = yoffs[j] + ty->nnz;
         lx[j] = {make_lin_params(G[j]->LX, tx->dims, 0), tx->d_idx, tx->d_val, tx->nnz};
         ly[j] = {make_lin_params(G[j]->LY, ty->dims, 1), ty->d_idx, ty->d_val, ty->nnz};
-        bp[j] = {G[j]->LX.ncbits, G[j]->LY.nfbits, G[j]->light_max};
+        bp[j] = {G[j]->LX.ncbits, G[j]->LY.nfbits, G[j]->light_max, col_words};
+        col_words += G[j]->LY.nfbits >= 38 ? 1ull << 33 : ((1ull << G[j]->LY.nfbits) + 31) >> 5;
     }
     const uint64_t nx = xoffs[g], ny = yoffs[g];
+    // Column ranks through presence bits (and a prefix of their words) where
+    // these take at most 64 B per Y nonzero, or 4 MiB, and a sixteenth of the
+    // memory left; by sorting the free indices otherwise.  For 1.55e5 entries
+    // over 2^24 free indices the scan and the lookups take 24 us (ncu) where the
+    // sort, its unique and the searches took 60; for 1e7 entries over 300, 42
+    // against 600.  The scan's time grows with the space (the bound keeps its
+    // bytes within a few times those of the sort's passes over Y), and the
+    // memory stays below the sort's two buffers except in the 4 MiB allowance.
+    const bool col_bits = col_words * 8 <= std::min(std::max<uint64_t>(64 * ny, 4ull << 20), A.available() / 16);
     DBuf<BLin> d_lx(A, g, s), d_ly(A, g, s);
     DBuf<BPrep> d_bp(A, g, s);
     DBuf<BatchJob> d_acc(A, g, s);
     DBuf<uint64_t> d_xoffs(A, g + 1, s), d_yoffs(A, g + 1, s);
-    DBuf<unsigned int> d_jerr(A, g, s), d_ydup(A, g, s);
-    // 0 ncols, 1 nruns, 2 nrows, 3 heavy rows, 4 light rows, 5 light units, 6 largest unit output,
-    // 7 stream rows, 8 heavy + stream rows, 9..11 shard row range and products
-    DBuf<uint64_t> cnts(A, 16, s);
+    // what starts at zero, cleared at once: the counters (kCnt*), the jobs'
+    // error and repeated-coordinate words, the scans' flags, the presence bits
+    const uint64_t zf_y = scan_flag_words(ny), zf_c = col_bits ? scan_flag_words(col_words) : 0,
+                   zf_x = scan_flag_words(nx);
+    const uint64_t zwords = 2 * kCnts + 2 * (uint64_t)g + zf_y + zf_c + 4 * zf_x + (col_bits ? col_words : 0);
+    DBuf<uint32_t> zero(A, zwords, s);
+    uint64_t *const cnts = reinterpret_cast<uint64_t *>(zero.get());
+    unsigned int *const d_jerr = zero.get() + 2 * kCnts, *const d_ydup = d_jerr + g;
+    uint32_t *const flags_y = d_ydup + g, *const flags_c = flags_y + zf_y, *const flags_x = flags_c + zf_c;
+    uint32_t *const ybits = col_bits ? flags_x + 4 * zf_x : nullptr;
+    // the scans' sums (one buffer: the scans follow one another on the stream)
+    DBuf<uint64_t> scan_vals(A, std::max({scan_value_words<1>(ny), col_bits ? scan_value_words<1>(col_words) : 0,
+                                          scan_value_words<4>(nx)}), s);
+    auto scan_state = [&](uint32_t *flags) { return ScanState{flags, scan_vals.get(), ctx->d_flag}; };
     h2d(d_lx.get(), lx.data(), g, s);
     h2d(d_ly.get(), ly.data(), g, s);
     h2d(d_bp.get(), bp.data(), g, s);
     h2d(d_xoffs.get(), xoffs.data(), g + 1, s);
     h2d(d_yoffs.get(), yoffs.data(), g + 1, s);
-    GS_CUDA(cudaMemsetAsync(d_jerr.get(), 0, 4 * g, s));
-    GS_CUDA(cudaMemsetAsync(d_ydup.get(), 0, 4 * g, s));
-    GS_CUDA(cudaMemsetAsync(cnts.get(), 0, 128, s));
+    GS_CUDA(cudaMemsetAsync(zero.get(), 0, 4 * zwords, s));
     GS_CUDA(cudaMemsetAsync(ctx->d_flag, 0, 4 * 4, s));
     bst.bytes_h2d += (sizeof(BLin) * 2 + sizeof(BPrep) + 16) * g;
 
@@ -796,27 +615,27 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     DBuf<uint32_t> rank(A, nyb, s);
     DBuf<uint64_t> cols(A, nyb, s), run_key(A, nyb, s);
     DBuf<uint32_t> run_start(A, ny + 1, s);
-    {
-        DBuf<uint8_t> flag(A, nyb, s);
+    if (col_bits) {
+        launch_y_runs(ykeys, ny, kby, d_bp, run_key, run_start, cnts, d_ydup, ybits, nullptr, scan_state(flags_y), s);
+        DBuf<uint32_t> wpre(A, col_words, s);
+        launch_col_table(ybits, col_words, d_bp, g, wpre, cols, cnts, scan_state(flags_c), s);
+        launch_y_ranks(ykeys, ny, kby, d_bp, g, ybits, wpre, cnts, rank, d_acc, ctx->d_flag, s);
+    } else {
         DBuf<uint64_t> yf0(A, nyb, s), yf1(A, nyb, s);
-        if (ny) {
-            k_by_split<<<grid_for(ny), kThreads, 0, s>>>(ykeys, ny, kby, d_bp, flag, yf0, d_ydup);
-            count_launch();
-            GS_CUDA(cudaGetLastError());
-        }
+        launch_y_runs(ykeys, ny, kby, d_bp, run_key, run_start, cnts, d_ydup, nullptr, yf0, scan_state(flags_y), s);
         int which = 0;
         sort_keys(A, ny, yf0, yf1, kby + jb, &which, s);
         uint64_t *sorted = which ? yf1.get() : yf0.get();
         uint64_t *uniq = which ? yf0.get() : yf1.get();
         if (ny) {
             size_t tmp = 0;
-            GS_CUDA(cub::DeviceSelect::Unique(nullptr, tmp, sorted, uniq, cnts.get() + 0, (int)ny, s));
+            GS_CUDA(cub::DeviceSelect::Unique(nullptr, tmp, sorted, uniq, cnts + kCntCols, (int)ny, s));
             DBuf<uint8_t> t(A, tmp, s);
-            GS_CUDA(cub::DeviceSelect::Unique(t.get(), tmp, sorted, uniq, cnts.get() + 0, (int)ny, s));
-            k_bcols<<<grid_for(ny), kThreads, 0, s>>>(uniq, cnts.get() + 0, kby, cols);
+            GS_CUDA(cub::DeviceSelect::Unique(t.get(), tmp, sorted, uniq, cnts + kCntCols, (int)ny, s));
+            k_bcols<<<grid_for(ny), kThreads, 0, s>>>(uniq, cnts + kCntCols, kby, cols);
             count_launch();
         }
-        k_bjobs<<<grid_for(g), kThreads, 0, s>>>(uniq, cnts.get() + 0, kby, g, d_bp, d_acc);
+        k_bjobs<<<grid_for(g), kThreads, 0, s>>>(uniq, cnts + kCntCols, kby, g, d_bp, d_acc);
         count_launch();
         GS_CUDA(cudaGetLastError());
         if (ny) {
@@ -824,11 +643,6 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
             count_launch();
             GS_CUDA(cudaGetLastError());
         }
-        select_idx(A, flag, ny, run_start, cnts.get() + 1, s);
-        k_bruns<<<grid_for(ny + 1), kThreads, 0, s>>>(ykeys, kby, d_bp, run_start, cnts.get() + 1, ny, run_key,
-                                                       run_start);
-        count_launch();
-        GS_CUDA(cudaGetLastError());
     }
 
     // ---- X match, row table and unit planning ----
@@ -837,12 +651,10 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     DBuf<uint32_t> row_start(A, nx + 1, s);
     DBuf<uint64_t> row_xf(A, nxb, s), row_prod(A, nxb, s);
     DBuf<uint16_t> row_job(A, nxb, s);
-    DBuf<uint32_t> H(A, nxb, s), hc(A, nx + 1, s), units(A, 2 * nxb, s);
-    DBuf<uint64_t> lpre(A, nx + 1, s);
-    DBuf<uint32_t> mpre(A, nx + 1, s), row_runs(A, nxb, s), row_xi(A, nxb, s), SR(A, nxb, s), mrun(A, nxb, s);
+    DBuf<uint32_t> H(A, nxb, s), units(A, 2 * nxb, s);
+    DBuf<uint32_t> mpre(A, nx + 1, s), mrun(A, nxb, s), row_xi(A, nxb, s), SR(A, nxb, s);
     DBuf<uint64_t> sprefix(A, nx + 1, s);
     DBuf<uint32_t> row_nnz(A, nxb, s);
-    GS_CUDA(cudaMemsetAsync(row_nnz.get(), 0, 4 * nxb, s));
     // heavy rows' kept column bitmaps: words of every heavy row and of the
     // dense ones only, their word offsets, each row's smallest rank
     const bool keep_bm = ctx->keep_row_bitmaps != 0;
@@ -852,99 +664,76 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         bm_w_all.reset(A, nxb, s);
         bm_w_dense.reset(A, nxb, s);
         row_rb.reset(A, nxb, s);
-        bm_off_all.reset(A, nx + 1, s);
-        bm_off_dense.reset(A, nx + 1, s);
+        bm_off_all.reset(A, nxb, s);
+        bm_off_dense.reset(A, nxb, s);
     }
-    {
-        DBuf<uint8_t> rflag(A, nxb, s);
-        if (nx) {
-            k_bmatch<<<grid_for(nx), kThreads, 0, s>>>(xkeys, nx, kbx, kby, d_bp, run_key, run_start,
-                                                        cnts.get() + 1, pos, cnt, rflag);
-            count_launch();
-            GS_CUDA(cudaGetLastError());
-        }
-        // 64-bit accumulation: a group's matched products can pass 2^32
-        cub::TransformInputIterator<uint64_t, CastU64, const uint32_t *> cit(cnt.get(), CastU64());
-        prefix_sum(A, cit, xprefix.get(), nx, s);
-        cub::TransformInputIterator<uint32_t, NonZero, const uint32_t *> mit(cnt.get(), NonZero());
-        prefix_sum(A, mit, mpre.get(), nx, s);
-        DBuf<uint32_t> rsx(A, nxb, s);
-        select_idx(A, rflag, nx, rsx, cnts.get() + 2, s);
-        rflag.release();
-        DBuf<uint8_t> heavy(A, nxb, s), lnz(A, nxb, s), sflag(A, nxb, s), brk(A, nxb, s);
-        DBuf<uint64_t> lp(A, nxb, s);
-        GS_CUDA(cudaMemsetAsync(row_prod.get(), 0, 8 * nxb, s));
-        k_brows<<<grid_for(nx + 1), kThreads, 0, s>>>(xkeys, kbx, d_bp, rsx, cnts.get() + 2, nx, xprefix, mpre,
-                                                       row_start, row_xf, row_job, row_prod, row_runs, row_xi);
+    if (nx) {
+        DBuf<uint8_t> rflag(A, nx, s), row_class(A, nx, s);
+        DBuf<uint32_t> mrow(A, nx, s), row_k0(A, nx + 1, s), L(A, nx, s), lbrk(A, nx, s);
+        DBuf<uint64_t> lpre(A, nx, s);
+        k_bmatch<<<grid_for(nx), kThreads, 0, s>>>(xkeys, nx, kbx, kby, d_bp, run_key, run_start, cnts + kCntRuns,
+                                                    pos, cnt, rflag);
         count_launch();
         GS_CUDA(cudaGetLastError());
+        RowArrays ra{};
+        ra.xprefix = xprefix;
+        ra.mpre = mpre;
+        ra.mrun = mrun;
+        ra.mrow = mrow;
+        ra.row_start = row_start;
+        ra.row_k0 = row_k0;
+        ra.row_xf = row_xf;
+        ra.row_job = row_job;
+        ra.row_prod = row_prod;
+        ra.row_class = row_class;
+        ra.row_nnz = row_nnz;
+        ra.row_xi = row_xi;
+        ra.H = H;
+        ra.SR = SR;
+        ra.L = L;
+        ra.sprefix = sprefix;
+        ra.lpre = lpre;
+        ra.lbrk = lbrk;
+        ra.units = units;
+        launch_x_rows(xkeys, nx, kbx, d_bp, cnt, rflag, ra, cnts, scan_state(flags_x), s);
         const uint64_t *range = nullptr;
         if (nshards > 1) {
-            DBuf<uint64_t> rp(A, nx + 1, s);
-            prefix_sum(A, row_prod.get(), rp.get(), nx, s);
-            k_shard_range<<<1, 32, 0, s>>>(rp, cnts.get() + 2, shard, nshards, cnts.get() + 9);
+            k_shard_range<<<1, 32, 0, s>>>(xprefix, row_start, cnts + kCntRows, shard, nshards, cnts + kCntRange,
+                                           ctx->d_flag);
             count_launch();
             GS_CUDA(cudaGetLastError());
-            range = cnts.get() + 9;
+            range = cnts + kCntRange;
         }
-        if (nx) {
-            k_bclass<<<grid_for(nx), kThreads, 0, s>>>(cnt, mpre, mrun, row_prod, row_runs, row_job, d_bp, d_ydup, cnts.get() + 2,
-                                                        range, nx, heavy, lnz, sflag, brk, lp, row_nnz);
-            count_launch();
-            GS_CUDA(cudaGetLastError());
-        }
-        select_idx(A, sflag, nx, SR, cnts.get() + 7, s);
-        {
-            DBuf<uint64_t> sprod(A, nxb, s);
-            if (nx) {
-                k_sprod<<<grid_for(nx), kThreads, 0, s>>>(SR, cnts.get() + 7, nx, row_prod, sprod);
-                count_launch();
-                GS_CUDA(cudaGetLastError());
-            }
-            prefix_sum(A, sprod.get(), sprefix.get(), nx, s);
-        }
+        launch_row_classes(nx, d_bp, d_ydup, range, ra, cnts, scan_state(flags_x + zf_x), s);
         mark(3);
-        prefix_sum(A, lp.get(), lpre.get(), nx, s);
-        cub::TransformInputIterator<uint32_t, CastU32, const uint8_t *> hit(heavy.get(), CastU32());
-        prefix_sum(A, hit, hc.get(), nx, s);
-        select_idx(A, heavy, nx, H, cnts.get() + 3, s);
-        DBuf<uint32_t> bc(A, nx + 1, s), B(A, nxb, s);
-        cub::TransformInputIterator<uint32_t, CastU32, const uint8_t *> bit(brk.get(), CastU32());
-        prefix_sum(A, bit, bc.get(), nx, s);
-        select_idx(A, brk, nx, B, cnts.get() + 8, s);
-        DBuf<uint32_t> L(A, nxb, s), S(A, nxb, s);
-        select_idx(A, lnz, nx, L, cnts.get() + 4, s);
-        if (nx) {
-            k_bstart<<<grid_for(nx), kThreads, 0, s>>>(L, cnts.get() + 4, lpre, bc,
-                                                        light_bin, nx, heavy);
-            count_launch();
-            GS_CUDA(cudaGetLastError());
-        }
-        select_idx(A, heavy, nx, S, cnts.get() + 5, s);  // `heavy` now holds the unit-start flags
-        k_bunits<<<grid_for(nx), kThreads, 0, s>>>(L, S, cnts, B, bc, units);
-        count_launch();
-        GS_CUDA(cudaGetLastError());
+        launch_light_units(nx, light_bin, ra, cnts, scan_state(flags_x + 2 * zf_x), s);
         if (keep_bm) {
-            launch_heavy_spans(H, cnts.get() + 3, nx, nx, row_start, pos, cnt, rank, row_prod, bm_w_all, bm_w_dense,
-                               row_rb, s);
-            exclusive_scan_u32_to_u64(A, bm_w_all, bm_off_all, nx, s);
-            exclusive_scan_u32_to_u64(A, bm_w_dense, bm_off_dense, nx, s);
+            DBuf<uint32_t> row_mx(A, nx, s);
+            GS_CUDA(cudaMemsetAsync(row_rb.get(), 0xff, 4 * nx, s));
+            GS_CUDA(cudaMemsetAsync(row_mx.get(), 0, 4 * nx, s));
+            launch_heavy_bitmaps(nx, pos, cnt, rank, ra, row_rb, row_mx, bm_w_all, bm_w_dense, bm_off_all,
+                                 bm_off_dense, cnts, scan_state(flags_x + 3 * zf_x), s);
         }
+    } else {
+        GS_CUDA(cudaMemsetAsync(xprefix.get(), 0, 8, s));
+        GS_CUDA(cudaMemsetAsync(mpre.get(), 0, 4, s));
+        GS_CUDA(cudaMemsetAsync(row_start.get(), 0, 4, s));
+        mark(3);
     }
-    uint64_t hc_cnt[16];
+    uint64_t hc_cnt[kCnts];
     std::vector<unsigned int> jerr(g);
     uint64_t ir = 0;
-    d2h(hc_cnt, cnts.get(), 16, s);
-    d2h(jerr.data(), d_jerr.get(), g, s);
+    unsigned int herr = 0;
+    d2h(hc_cnt, cnts, kCnts, s);
+    d2h(jerr.data(), d_jerr, g, s);
     d2h(&ir, xprefix.get() + nx, 1, s);
-    uint64_t bm_words_all = 0, bm_words_dense = 0;
-    if (keep_bm) {
-        d2h(&bm_words_all, bm_off_all.get() + nx, 1, s);
-        d2h(&bm_words_dense, bm_off_dense.get() + nx, 1, s);
-    }
+    d2h(&herr, ctx->d_flag, 1, s);
     GS_CUDA(cudaStreamSynchronize(s));
-    const uint64_t nrows = hc_cnt[2], nh = hc_cnt[3], nu = hc_cnt[5], nsr = hc_cnt[7];
-    if (nshards > 1) ir = hc_cnt[11];  // the shard's products
+    GS_REQUIRE(!(herr & kScanErr), GSPARC_EINTERNAL, "a prefix sum's or the radix sort's look-back gave up");
+    const uint64_t bm_words_all = hc_cnt[kCntBmAll], bm_words_dense = hc_cnt[kCntBmDense];
+    const uint64_t nrows = hc_cnt[kCntRows], nh = hc_cnt[kCntHeavy], nu = hc_cnt[kCntUnits],
+                   nsr = hc_cnt[kCntStream];
+    if (nshards > 1) ir = hc_cnt[kCntRange + 2];  // the shard's products
     bst.ir_nnz += ir;
     bst.rows += nrows;
     bst.heavy_rows += nh;
@@ -952,25 +741,20 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
 
     // heavy rows largest first (H itself stays in row order for chunk planning)
     DBuf<uint32_t> H2;
-    DBuf<uint64_t> hp0, hp1;
     const uint32_t *Hs = H.get();
     if (nh > 1) {
-        hp0.reset(A, nh, s);
-        hp1.reset(A, nh, s);
+        DBuf<uint8_t> hp0(A, nh, s), hp1(A, nh, s);
         H2.reset(A, nh, s);
-        k_gather_prod<<<grid_for(nh), kThreads, 0, s>>>(H, nh, row_prod, hp0);
+        k_heavy_sizes<<<grid_for(nh), kThreads, 0, s>>>(H, nh, row_prod, hp0);
         count_launch();
         GS_CUDA(cudaGetLastError());
-        const int bits = std::max(1, 64 - __builtin_clzll(std::max<uint64_t>(ir, 1)));
         size_t tmp = 0;
         GS_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp, hp0.get(), hp1.get(), H.get(), H2.get(),
-                                                          (int)nh, 0, bits, s));
+                                                          (int)nh, 0, 8, s));
         DBuf<uint8_t> t(A, tmp, s);
         GS_CUDA(cub::DeviceRadixSort::SortPairsDescending(t.get(), tmp, hp0.get(), hp1.get(), H.get(), H2.get(),
-                                                          (int)nh, 0, bits, s));
+                                                          (int)nh, 0, 8, s));
         Hs = H2.get();
-        hp0.release();
-        hp1.release();
     }
 
     // ---- symbolic pass ----
@@ -1018,13 +802,18 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         hbm.reset(A, words, s);
         aa.hbm = hbm;
         aa.row_bmoff = *bm_off;
+        aa.row_bmw = bm_off == &bm_off_all ? bm_w_all : bm_w_dense;
         aa.row_rb = row_rb;
         bst.kept_bitmap_bytes += words * 4;
     }
-    bm_w_all.release();
-    bm_w_dense.release();
-    if (bm_off != &bm_off_all) bm_off_all.release();
-    if (bm_off != &bm_off_dense) bm_off_dense.release();
+    if (bm_off != &bm_off_all) {
+        bm_off_all.release();
+        bm_w_all.release();
+    }
+    if (bm_off != &bm_off_dense) {
+        bm_off_dense.release();
+        bm_w_dense.release();
+    }
     const int ghs = std::max(1, ctx->sm_count * heavy_blocks_per_sm(false));
     const int gh = std::max(1, ctx->sm_count * heavy_blocks_per_sm(true));
     const int gl = std::max(1, ctx->sm_count * light_blocks_per_sm());
@@ -1042,26 +831,19 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     }
     exclusive_scan_u32_to_u64(A, row_nnz, row_off, nrows, s);
     DBuf<JobOut> d_jo(A, g + 1, s);
-    k_bjobout<<<grid_for(g + 1), kThreads, 0, s>>>(row_job, nrows, row_off, xprefix, hc, d_xoffs, g, d_jo);
+    const UnitLists ul{units, nu, H, nh, SR, nsr};
+    k_after_counts<<<grid_for(std::max<uint64_t>(nu + nh + nsr, (uint64_t)g + 1)), kThreads, 0, s>>>(
+        ul, row_off, row_job, nrows, xprefix, d_xoffs, g, d_jo, cnts + kCntMaxUnit);
     count_launch();
     GS_CUDA(cudaGetLastError());
-    GS_CUDA(cudaMemsetAsync(cnts.get() + 6, 0, 8, s));
-    const UnitLists ul{units, nu, H, nh, SR, nsr};
-    if (nu + nh + nsr) {
-        k_unit_max<<<grid_for(nu + nh + nsr), kThreads, 0, s>>>(ul, row_off, cnts.get() + 6);
-        count_launch();
-        GS_CUDA(cudaGetLastError());
-    }
     std::vector<JobOut> jo(g + 1);
-    unsigned int herr = 0;
     uint64_t max_unit = 0;
     d2h(jo.data(), d_jo.get(), g + 1, s);
     d2h(&herr, ctx->d_flag, 1, s);
-    d2h(&max_unit, cnts.get() + 6, 1, s);
+    d2h(&max_unit, cnts + kCntMaxUnit, 1, s);
     GS_CUDA(cudaStreamSynchronize(s));
     bst.bytes_d2h += sizeof(JobOut) * (g + 1) + 64 + 4 * g + 8;
     GS_REQUIRE(!(herr & 2u), GSPARC_EINTERNAL, "light unit over capacity");
-    GS_REQUIRE(!(herr & 8u), GSPARC_EINTERNAL, "radix sort look-back gave up");
     const uint64_t ntot = jo[g].out_off;
     bst.nnz += ntot;
     mark(4);
@@ -1212,6 +994,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
             keep->hbm = std::move(hbm);
             keep->row_rb = std::move(row_rb);
             keep->row_bmoff = std::move(*bm_off);
+            keep->row_bmw = std::move(bm_off == &bm_off_all ? bm_w_all : bm_w_dense);
         }
         keep->chunks.clear();
         for (auto &c : chunks) keep->chunks.push_back({c.lu0, c.lu1, c.h0, c.h1, c.s0, c.s1, c.first, c.n});

@@ -1,0 +1,86 @@
+// rows.h -- the planning kernels of a group (rows.cu): Y's run and column
+// tables, X's rows, the row classes and the unit lists.
+#pragma once
+
+#include "kernels.cuh"
+#include "scan.cuh"
+
+namespace gs {
+
+// Per-job constants of the planning kernels.
+struct BPrep {
+    int x_ncbits;
+    int y_nfbits;
+    uint64_t light_max;  // rows with more products go to the windowed accumulator
+    uint64_t col_word0;  // first word of the job's Y free indices in the presence bits
+};
+
+// Device counters of a group.
+enum {
+    kCntCols = 0,     // distinct Y free indices
+    kCntRuns = 1,     // runs of Y
+    kCntRows = 2,
+    kCntHeavy = 3,
+    kCntLight = 4,    // light rows
+    kCntUnits = 5,    // light units
+    kCntMaxUnit = 6,  // largest unit output
+    kCntStream = 7,
+    kCntRange = 9,    // 9..11 shard row range and products
+    kCntBmAll = 12,   // words of every kept bitmap
+    kCntBmDense = 13, // words of the dense rows' kept bitmaps
+    kCnts = 16
+};
+
+constexpr uint8_t kRowNone = 0, kRowLight = 1, kRowStream = 2, kRowHeavy = 3;
+
+// Sorted Y keys -> run table (run_key, run_start with the closing entry, count
+// in cnts), ydup per job; marks every entry's free index in the presence bits
+// (bits null: writes the prefixed free index to yfk instead).
+void launch_y_runs(const uint64_t *ykeys, uint64_t ny, int kby, const BPrep *jobs, uint64_t *run_key,
+                   uint32_t *run_start, uint64_t *cnts, unsigned int *ydup, uint32_t *bits, uint64_t *yfk,
+                   const ScanState &st, cudaStream_t s);
+// Presence bits -> distinct free indices of every job (cols, ascending) and
+// the number of distinct ones before every word (wpre).
+void launch_col_table(const uint32_t *bits, uint64_t nwords, const BPrep *jobs, int g, uint32_t *wpre, uint64_t *cols,
+                      uint64_t *cnts, const ScanState &st, cudaStream_t s);
+// Column rank of every Y entry inside its job, and the jobs' column ranges.
+void launch_y_ranks(const uint64_t *ykeys, uint64_t ny, int kby, const BPrep *jobs, int g, const uint32_t *bits,
+                    const uint32_t *wpre, const uint64_t *cnts, uint32_t *rank, BatchJob *acc,
+                    const unsigned int *err, cudaStream_t s);
+
+struct RowArrays {
+    uint64_t *xprefix;   // [nx + 1] matched products before every X nonzero
+    uint32_t *mpre;      // [nx + 1] matched X nonzeros before every one
+    uint32_t *mrun;      // [matched] the matched X nonzeros
+    uint32_t *mrow;      // [matched] their rows
+    uint32_t *row_start; // [nrows + 1]
+    uint32_t *row_k0;    // [nrows + 1] first matched X nonzero (index into mrun)
+    uint64_t *row_xf;    // [nrows]
+    uint16_t *row_job;   // [nrows]
+    uint64_t *row_prod;  // [nrows]
+    uint8_t *row_class;  // [nrows]
+    uint32_t *row_nnz;   // [nrows] stream rows: their products; 0 otherwise
+    uint32_t *row_xi;    // [nrows] stream rows: their matched X nonzero
+    uint32_t *H, *SR, *L;  // heavy, stream and light rows, in row order
+    uint64_t *sprefix;   // [stream + 1] products before every stream row
+    uint64_t *lpre;      // [light] products of the light rows before each one
+    uint32_t *lbrk;      // [light] heavy and stream rows before each light row
+    uint32_t *units;     // light units: row pairs
+};
+// Match of every X nonzero -> prefix sums, matched list and rows.
+void launch_x_rows(const uint64_t *xkeys, uint64_t nx, int kbx, const BPrep *jobs, const uint32_t *cnt,
+                   const uint8_t *row_flag, const RowArrays &r, uint64_t *cnts, const ScanState &st, cudaStream_t s);
+// Row classes, their lists and product prefixes (rows outside `range` get no class).
+void launch_row_classes(uint64_t nx, const BPrep *jobs, const unsigned int *ydup, const uint64_t *range,
+                        const RowArrays &r, uint64_t *cnts, const ScanState &st, cudaStream_t s);
+// Light units of at most bin + light_max products.
+void launch_light_units(uint64_t nx, uint64_t bin, const RowArrays &r, uint64_t *cnts, const ScanState &st,
+                        cudaStream_t s);
+// Kept bitmaps: rank span of every heavy row, its words with all / only dense
+// rows kept (w_*, by row), their word offsets (off_*, by row) and totals.
+// row_rb must hold all ones and row_mx zeros for every heavy row.
+void launch_heavy_bitmaps(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, const uint32_t *yrank,
+                          const RowArrays &r, uint32_t *row_rb, uint32_t *row_mx, uint32_t *w_all, uint32_t *w_dense,
+                          uint64_t *off_all, uint64_t *off_dense, uint64_t *cnts, const ScanState &st, cudaStream_t s);
+
+}  // namespace gs

@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
         const uint32_t row = a.units[u];
         const uint32_t xs = a.row_start[row], xe = a.row_start[row + 1];
         // words of the row's kept column bitmap (0: none, the windows mark their columns)
-        const uint32_t nwr = a.row_bmoff ? (uint32_t)(a.row_bmoff[row + 1] - a.row_bmoff[row]) : 0u;
+        const uint32_t nwr = a.row_bmoff ? a.row_bmw[row] : 0u;
         if (tid == 0) {  // read after the barriers of block_min_u32 below
             int y_nfbits;
             const uint64_t *cols;
@@ -746,44 +746,6 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
     }
 }
 
-// Rank span of every heavy row: a warp per row (grid-stride over H, whose
-// count is on the device); runs are sorted by rank, so a run's first and last
-// entries bound it.
-__global__ void k_hspan(const uint32_t *__restrict__ H, const uint64_t *__restrict__ nh,
-                        const uint32_t *__restrict__ row_start, const uint32_t *__restrict__ pos,
-                        const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ yrank,
-                        const uint64_t *__restrict__ row_prod, uint32_t *__restrict__ w_all,
-                        uint32_t *__restrict__ w_dense, uint32_t *__restrict__ row_rb) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    const uint64_t n = *nh;
-    for (uint64_t k = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += nwarps) {
-        const uint32_t row = H[k];
-        const uint32_t xs = row_start[row], xe = row_start[row + 1];
-        uint32_t mn = INF, mx = 0;
-        for (uint32_t i = xs + lane; i < xe; i += 32) {
-            const uint32_t c = cnt[i];
-            if (c) {
-                const uint32_t p = pos[i];
-                mn = min(mn, yrank[p]);
-                mx = max(mx, yrank[p + c - 1]);
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            mn = min(mn, __shfl_xor_sync(FULL, mn, o));
-            mx = max(mx, __shfl_xor_sync(FULL, mx, o));
-        }
-        if (lane == 0 && mn != INF) {
-            const uint64_t span = (uint64_t)mx - mn + 1;
-            const uint32_t words = (uint32_t)(((span + 127) >> 7) << 2);
-            w_all[row] = span <= kKeepBitsMax * row_prod[row] ? words : 0u;
-            w_dense[row] = span <= kKeepBitsPerProduct * row_prod[row] ? words : 0u;
-            row_rb[row] = mn;
-        }
-    }
-}
-
 size_t rowwin_smem(bool numeric) {
     const size_t words = (numeric ? (size_t)AW + MAXR : (size_t)NWORDS_SYM) + MAXR + (MAXR + 4) + MAXR + MAXR;
     return words * 4 + (numeric ? (size_t)CAP * 8 : 0);
@@ -816,23 +778,6 @@ void launch_heavy(const AccArgs &a, bool numeric, int grid, cudaStream_t s) {
         GS_CUDA(cudaFuncSetAttribute(k_rowwin<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         k_rowwin<false><<<grid, T, sm, s>>>(a);
     }
-    count_launch();
-    GS_CUDA(cudaGetLastError());
-}
-
-void launch_heavy_spans(const uint32_t *H, const uint64_t *nh, uint64_t nh_max, uint64_t nrows_max,
-                        const uint32_t *row_start, const uint32_t *pos, const uint32_t *cnt,
-                        const uint32_t *yrank, const uint64_t *row_prod, uint32_t *w_all, uint32_t *w_dense,
-                        uint32_t *row_rb, cudaStream_t s) {
-    if (nrows_max) {
-        GS_CUDA(cudaMemsetAsync(w_all, 0, sizeof(uint32_t) * nrows_max, s));
-        GS_CUDA(cudaMemsetAsync(w_dense, 0, sizeof(uint32_t) * nrows_max, s));
-    }
-    if (nh_max == 0) return;
-    constexpr int B = 256;
-    const uint64_t blocks = (nh_max * 32 + B - 1) / B;
-    k_hspan<<<(unsigned)std::min<uint64_t>(blocks, 4096), B, 0, s>>>(H, nh, row_start, pos, cnt, yrank, row_prod,
-                                                                     w_all, w_dense, row_rb);
     count_launch();
     GS_CUDA(cudaGetLastError());
 }
