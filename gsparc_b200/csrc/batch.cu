@@ -147,7 +147,8 @@ __global__ void k_bcols(const uint64_t *__restrict__ uniq, const uint64_t *__res
 
 // Per-job column table range inside the group's table.
 __global__ void k_bjobs(const uint64_t *__restrict__ uniq, const uint64_t *__restrict__ ncols_dev,
-                        int kby, int g, const BPrep *__restrict__ jobs, BatchJob *__restrict__ acc) {
+                        int kby, int g, const BPrep *__restrict__ jobs, const unsigned int *__restrict__ ydup,
+                        BatchJob *__restrict__ acc) {
     const uint64_t n = *ncols_dev;
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < g; j += gridDim.x * blockDim.x) {
         const uint64_t lo = lower_bound_dev<uint64_t>(uniq, 0, n, shl((uint64_t)j, kby));
@@ -155,6 +156,7 @@ __global__ void k_bjobs(const uint64_t *__restrict__ uniq, const uint64_t *__res
         BatchJob b;
         b.y_nfbits = jobs[j].y_nfbits;
         b.ncols = (uint32_t)(hi - lo);
+        b.ydup = ydup[j];
         b.cols_off = lo;
         acc[j] = b;
     }
@@ -245,16 +247,18 @@ __global__ void k_shard_range(const uint64_t *__restrict__ xprefix, const uint32
     }
 }
 
-// Sort key of the largest-first order of the heavy rows: the product count's
-// binary exponent and two mantissa bits, one 8-bit radix pass (the order only
-// balances the CTAs: a row within a fifth of the next is as good).
+// Sort key of the heavy rows' order (descending): rows of the windowed kernel
+// before narrow rows, largest first by the product count's binary exponent and
+// one mantissa bit, in one 8-bit radix pass (the order only balances the work:
+// a row within a third of the next is as good).
 __global__ void k_heavy_sizes(const uint32_t *__restrict__ H, uint64_t nh, const uint64_t *__restrict__ row_prod,
-                              uint8_t *__restrict__ hp) {
+                              const uint8_t *__restrict__ row_class, uint8_t *__restrict__ hp) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nh; k += stride) {
-        const uint64_t p = row_prod[H[k]] | 4u;
+        const uint64_t p = row_prod[H[k]] | 2u;
         const int e = 63 - __clzll((long long)p);
-        hp[k] = (uint8_t)((e << 2) | ((p >> (e - 2)) & 3u));
+        const bool narrow = row_class && row_class[H[k]] == kRowNarrow;
+        hp[k] = (uint8_t)((narrow ? 0 : 128) | (e << 1) | ((p >> (e - 1)) & 1u));
     }
 }
 
@@ -363,10 +367,11 @@ __global__ void k_chunk_bounds(const uint32_t *__restrict__ urow, const uint64_t
     }
 }
 
-// Sort key grouping heavy rows by chunk, largest first inside a chunk.
+// Sort key grouping heavy rows by chunk, inside a chunk the windowed kernel's
+// rows before the narrow rows, largest first.
 __global__ void k_heavy_chunk_keys(const uint32_t *__restrict__ Hs, uint64_t nh,
-                                   const uint64_t *__restrict__ row_prod, const uint64_t *__restrict__ info,
-                                   uint64_t K, uint64_t *__restrict__ keys) {
+                                   const uint64_t *__restrict__ row_prod, const uint8_t *__restrict__ row_class,
+                                   const uint64_t *__restrict__ info, uint64_t K, uint64_t *__restrict__ keys) {
     constexpr uint64_t kProdMask = (1ull << 44) - 1;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nh; k += stride) {
@@ -380,7 +385,8 @@ __global__ void k_heavy_chunk_keys(const uint32_t *__restrict__ Hs, uint64_t nh,
                 hi = mid;
         }
         const uint64_t p = row_prod[r];
-        keys[k] = (lo << 44) | (kProdMask - (p < kProdMask ? p : kProdMask));
+        const uint64_t narrow = row_class && row_class[r] == kRowNarrow;
+        keys[k] = (lo << 45) | (narrow << 44) | (kProdMask - (p < kProdMask ? p : kProdMask));
     }
 }
 
@@ -424,7 +430,8 @@ struct Times {
 // table, the match, the rows, the unit lists and the output offsets.
 struct GroupPlan {
     int g = 0;
-    uint64_t nx = 0, ny = 0, ntot = 0, nu = 0, nh = 0, nsr = 0;
+    uint64_t nx = 0, ny = 0, ntot = 0, nu = 0, nh = 0, nsr = 0, nnarrow = 0;
+    int sm_count = 148;
     int gl = 1, gh = 1, gs_grid = 1;
     AccArgs aa{};
     std::vector<uint64_t> job_first;  // g + 1 group-local output offsets
@@ -440,6 +447,9 @@ struct GroupPlan {
     DBuf<uint32_t> Hc;         // heavy rows grouped by chunk (several chunks only)
     DBuf<uint32_t> hbm, row_rb, row_bmw;  // heavy rows' kept column bitmaps (may be empty)
     DBuf<uint64_t> row_bmoff;
+    DBuf<uint32_t> nbm, unit_off, part_off;  // narrow rows (may be empty)
+    DBuf<float2> part;
+    DBuf<uint8_t> row_class;
     DBuf<unsigned int> flags;  // error bits, work counter, windows swept, spare
     struct Chunk {
         uint64_t lu0, lu1, h0, h1, s0, s1, first, n;
@@ -545,12 +555,12 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     // error and repeated-coordinate words, the scans' flags, the presence bits
     const uint64_t zf_y = scan_flag_words(ny), zf_c = col_bits ? scan_flag_words(col_words) : 0,
                    zf_x = scan_flag_words(nx);
-    const uint64_t zwords = 2 * kCnts + 2 * (uint64_t)g + zf_y + zf_c + 4 * zf_x + (col_bits ? col_words : 0);
+    const uint64_t zwords = 2 * kCnts + 2 * (uint64_t)g + zf_y + zf_c + 6 * zf_x + (col_bits ? col_words : 0);
     DBuf<uint32_t> zero(A, zwords, s);
     uint64_t *const cnts = reinterpret_cast<uint64_t *>(zero.get());
     unsigned int *const d_jerr = zero.get() + 2 * kCnts, *const d_ydup = d_jerr + g;
     uint32_t *const flags_y = d_ydup + g, *const flags_c = flags_y + zf_y, *const flags_x = flags_c + zf_c;
-    uint32_t *const ybits = col_bits ? flags_x + 4 * zf_x : nullptr;
+    uint32_t *const ybits = col_bits ? flags_x + 6 * zf_x : nullptr;
     // the scans' sums (one buffer: the scans follow one another on the stream)
     DBuf<uint64_t> scan_vals(A, std::max({scan_value_words<1>(ny), col_bits ? scan_value_words<1>(col_words) : 0,
                                           scan_value_words<4>(nx)}), s);
@@ -619,7 +629,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         launch_y_runs(ykeys, ny, kby, d_bp, run_key, run_start, cnts, d_ydup, ybits, nullptr, scan_state(flags_y), s);
         DBuf<uint32_t> wpre(A, col_words, s);
         launch_col_table(ybits, col_words, d_bp, g, wpre, cols, cnts, scan_state(flags_c), s);
-        launch_y_ranks(ykeys, ny, kby, d_bp, g, ybits, wpre, cnts, rank, d_acc, ctx->d_flag, s);
+        launch_y_ranks(ykeys, ny, kby, d_bp, g, ybits, wpre, cnts, rank, d_acc, d_ydup, ctx->d_flag, s);
     } else {
         DBuf<uint64_t> yf0(A, nyb, s), yf1(A, nyb, s);
         launch_y_runs(ykeys, ny, kby, d_bp, run_key, run_start, cnts, d_ydup, nullptr, yf0, scan_state(flags_y), s);
@@ -635,7 +645,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
             k_bcols<<<grid_for(ny), kThreads, 0, s>>>(uniq, cnts + kCntCols, kby, cols);
             count_launch();
         }
-        k_bjobs<<<grid_for(g), kThreads, 0, s>>>(uniq, cnts + kCntCols, kby, g, d_bp, d_acc);
+        k_bjobs<<<grid_for(g), kThreads, 0, s>>>(uniq, cnts + kCntCols, kby, g, d_bp, d_ydup, d_acc);
         count_launch();
         GS_CUDA(cudaGetLastError());
         if (ny) {
@@ -660,6 +670,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     const bool keep_bm = ctx->keep_row_bitmaps != 0;
     DBuf<uint32_t> bm_w_all, bm_w_dense, row_rb;
     DBuf<uint64_t> bm_off_all, bm_off_dense;
+    DBuf<uint8_t> row_class;
     if (keep_bm) {
         bm_w_all.reset(A, nxb, s);
         bm_w_dense.reset(A, nxb, s);
@@ -668,7 +679,8 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         bm_off_dense.reset(A, nxb, s);
     }
     if (nx) {
-        DBuf<uint8_t> rflag(A, nx, s), row_class(A, nx, s);
+        DBuf<uint8_t> rflag(A, nx, s);
+        row_class.reset(A, nx, s);
         DBuf<uint32_t> mrow(A, nx, s), row_k0(A, nx + 1, s), L(A, nx, s), lbrk(A, nx, s);
         DBuf<uint64_t> lpre(A, nx, s);
         k_bmatch<<<grid_for(nx), kThreads, 0, s>>>(xkeys, nx, kbx, kby, d_bp, run_key, run_start, cnts + kCntRuns,
@@ -704,7 +716,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
             GS_CUDA(cudaGetLastError());
             range = cnts + kCntRange;
         }
-        launch_row_classes(nx, d_bp, d_ydup, range, ra, cnts, scan_state(flags_x + zf_x), s);
+        launch_row_classes(nx, d_bp, d_acc, range, ra, cnts, scan_state(flags_x + zf_x), s);
         mark(3);
         launch_light_units(nx, light_bin, ra, cnts, scan_state(flags_x + 2 * zf_x), s);
         if (keep_bm) {
@@ -739,13 +751,24 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     bst.heavy_rows += nh;
     bst.stream_rows += nsr;
 
+    // Narrow rows: units of about `slice` products (some 24 CTAs' worth an SM,
+    // so that the last ones end together), their columns' marks and the partial
+    // sums of rows of several units.  Where these do not fit a sixteenth of the
+    // memory left, the windowed kernel takes the rows.
+    const uint64_t slice = std::min<uint64_t>(std::max<uint64_t>(ir / ((uint64_t)ctx->sm_count * 24), kNarrowSlice),
+                                              1ull << 20);
+    const uint64_t narrow_cols = hc_cnt[kCntNarrowCols], nbm_words = hc_cnt[kCntNarrow] * (kNarrowCols / 32),
+                   nparts = 2 * (ir / slice) * narrow_cols;
+    const uint64_t nnarrow = 4 * nbm_words + 8 * nparts <= A.available() / 16 ? hc_cnt[kCntNarrow] : 0;
+    const uint8_t *narrow_class = nnarrow ? row_class.get() : nullptr;
+
     // heavy rows largest first (H itself stays in row order for chunk planning)
     DBuf<uint32_t> H2;
     const uint32_t *Hs = H.get();
     if (nh > 1) {
         DBuf<uint8_t> hp0(A, nh, s), hp1(A, nh, s);
         H2.reset(A, nh, s);
-        k_heavy_sizes<<<grid_for(nh), kThreads, 0, s>>>(H, nh, row_prod, hp0);
+        k_heavy_sizes<<<grid_for(nh), kThreads, 0, s>>>(H, nh, row_prod, narrow_class, hp0);
         count_launch();
         GS_CUDA(cudaGetLastError());
         size_t tmp = 0;
@@ -784,6 +807,23 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     aa.row_xi = row_xi;
     aa.err = ctx->d_flag;
     aa.heavy_cap = ctx->heavy_window_cap;
+    DBuf<uint32_t> nbm, unit_off, part_off;
+    DBuf<float2> part;
+    if (nnarrow) {
+        nbm.reset(A, nbm_words, s);
+        unit_off.reset(A, nh + 1, s);
+        part_off.reset(A, nh, s);
+        part.reset(A, std::max<uint64_t>(nparts, 1), s);
+        GS_CUDA(cudaMemsetAsync(nbm.get(), 0, 4 * nbm_words, s));
+        launch_narrow_units(Hs, (uint32_t)nh, row_class, row_prod, slice, unit_off, part_off,
+                            scan_state(flags_x + 4 * zf_x), s);
+        aa.row_class = row_class;
+        aa.unit_off = unit_off;
+        aa.part_off = part_off;
+        aa.nbm = nbm;
+        aa.part = part;
+        aa.narrow_cols = (uint32_t)narrow_cols;
+    }
     // Kept bitmaps take at most an eighth of the memory left (the rest is for
     // the output chunks): those of the heavy rows of at most kKeepBitsMax bits
     // per product if they fit, else of the dense rows (at most
@@ -826,8 +866,14 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         launch_light(b, false, (int)std::min<uint64_t>(gl, std::max<uint64_t>(1, nu)), s);
         b.units = Hs;
         b.nunits = (uint32_t)nh;
-        GS_CUDA(cudaMemsetAsync(ctx->d_flag + 1, 0, 4, s));
-        launch_heavy(b, false, (int)std::min<uint64_t>(ghs, std::max<uint64_t>(1, nh)), s);
+        if (nh > nnarrow) {
+            GS_CUDA(cudaMemsetAsync(ctx->d_flag + 1, 0, 4, s));
+            launch_heavy(b, false, (int)std::min<uint64_t>(ghs, std::max<uint64_t>(1, nh)), s);
+        }
+        if (nnarrow) {
+            GS_CUDA(cudaMemsetAsync(ctx->d_flag + 1, 0, 4, s));
+            launch_narrow(b, false, ctx->sm_count, s);
+        }
     }
     exclusive_scan_u32_to_u64(A, row_nnz, row_off, nrows, s);
     DBuf<JobOut> d_jo(A, g + 1, s);
@@ -929,10 +975,10 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
             // heavy rows grouped by chunk (stable in the largest-first order)
             DBuf<uint64_t> hk0(A, nh, s), hk1(A, nh, s);
             Hc.reset(A, nh, s);
-            k_heavy_chunk_keys<<<grid_for(nh), kThreads, 0, s>>>(Hs, nh, row_prod, cinfo, K, hk0);
+            k_heavy_chunk_keys<<<grid_for(nh), kThreads, 0, s>>>(Hs, nh, row_prod, aa.row_class, cinfo, K, hk0);
             count_launch();
             GS_CUDA(cudaGetLastError());
-            const int bits = 44 + ceil_log2(K);
+            const int bits = 45 + ceil_log2(K);
             size_t tmp = 0;
             GS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, hk0.get(), hk1.get(), Hs, Hc.get(), (int)nh, 0,
                                                     bits, s));
@@ -949,6 +995,9 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         }
     }
     bst.chunks += chunks.size();
+    if (nnarrow && Hchunk != Hs)  // the chunks' own order
+        launch_narrow_units(Hchunk, (uint32_t)nh, row_class, row_prod, slice, unit_off, part_off,
+                            scan_state(flags_x + 5 * zf_x), s);
 
     if (keep) {
         // a plan keeps what the numeric pass needs and stops here
@@ -998,6 +1047,15 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         }
         keep->chunks.clear();
         for (auto &c : chunks) keep->chunks.push_back({c.lu0, c.lu1, c.h0, c.h1, c.s0, c.s1, c.first, c.n});
+        if (nnarrow) {
+            keep->nnarrow = nnarrow;
+            keep->nbm = std::move(nbm);
+            keep->unit_off = std::move(unit_off);
+            keep->part_off = std::move(part_off);
+            keep->part = std::move(part);
+            keep->row_class = std::move(row_class);
+        }
+        keep->sm_count = ctx->sm_count;
         keep->flags.reset(A, 4, s);
         GS_CUDA(cudaMemsetAsync(keep->flags.get(), 0, 16, s));
         keep->aa = aa;  // the moved buffers keep their device addresses
@@ -1092,8 +1150,16 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         launch_light(b, true, (int)std::min<uint64_t>(gl, std::max<uint64_t>(1, b.nunits)), sc);
         b.units = Hchunk + c.h0;
         b.nunits = (uint32_t)(c.h1 - c.h0);
-        GS_CUDA(cudaMemsetAsync(counter, 0, 4, sc));
-        launch_heavy(b, true, (int)std::min<uint64_t>(gh, std::max<uint64_t>(1, b.nunits)), sc);
+        if (nh > nnarrow) {
+            GS_CUDA(cudaMemsetAsync(counter, 0, 4, sc));
+            launch_heavy(b, true, (int)std::min<uint64_t>(gh, std::max<uint64_t>(1, b.nunits)), sc);
+        }
+        if (nnarrow) {
+            b.unit_off += c.h0;
+            b.part_off += c.h0;
+            GS_CUDA(cudaMemsetAsync(counter, 0, 4, sc));
+            launch_narrow(b, true, ctx->sm_count, sc);
+        }
         b.units = SR.get() + c.s0;
         b.nunits = (uint32_t)(c.s1 - c.s0);
         b.sprefix = sprefix.get() + c.s0;
@@ -1471,8 +1537,16 @@ void plan_execute(gsparc_plan *P, uint64_t chunk, uint64_t *keys, float *vals, u
     launch_light(b, true, (int)std::min<uint64_t>(gp.gl, std::max<uint64_t>(1, b.nunits)), s);
     b.units = gp.heavy_list() + c.h0;
     b.nunits = (uint32_t)(c.h1 - c.h0);
-    GS_CUDA(cudaMemsetAsync(gp.flags.get() + 1, 0, 4, s));
-    launch_heavy(b, true, (int)std::min<uint64_t>(gp.gh, std::max<uint64_t>(1, b.nunits)), s);
+    if (gp.nh > gp.nnarrow) {
+        GS_CUDA(cudaMemsetAsync(gp.flags.get() + 1, 0, 4, s));
+        launch_heavy(b, true, (int)std::min<uint64_t>(gp.gh, std::max<uint64_t>(1, b.nunits)), s);
+    }
+    if (gp.nnarrow) {
+        b.unit_off += c.h0;
+        b.part_off += c.h0;
+        GS_CUDA(cudaMemsetAsync(gp.flags.get() + 1, 0, 4, s));
+        launch_narrow(b, true, gp.sm_count, s);
+    }
     b.units = gp.SR.get() + c.s0;
     b.nunits = (uint32_t)(c.s1 - c.s0);
     b.sprefix = gp.sprefix.get() + c.s0;

@@ -69,6 +69,7 @@ void match_x(Arena &a, const uint64_t *xkeys, uint64_t nx, int x_ncbits, const Y
 struct BatchJob {
     int y_nfbits;       // the job's Y free bits (output key = x_f << y_nfbits | y_f)
     uint32_t ncols;     // the job's distinct Y free indices
+    uint32_t ydup;      // nonzero: the job's Y repeats a coordinate
     uint64_t cols_off;  // where the job's distinct Y free indices start in `cols`
 };
 
@@ -93,7 +94,7 @@ struct AccArgs {
     int y_nfbits;
     // single-run rows (stream path): the matched X nonzero of every such row,
     // and the product prefix over the listed rows (nunits + 1 entries)
-    const uint32_t *row_xi;
+    const uint32_t *row_xi;     // (of a narrow row: its number among the narrow rows)
     const uint64_t *sprefix;
     // work
     const uint32_t *units;     // light: pairs (r0, r1); heavy and stream: row ids
@@ -112,6 +113,14 @@ struct AccArgs {
     const uint64_t *row_bmoff;  // [nrows]
     const uint32_t *row_bmw;    // [nrows]
     const uint32_t *row_rb;     // [nrows]
+    // heavy lists hold the rows of the windowed kernel, then the narrow rows
+    // (narrow.cu; row_class null: none of those)
+    const uint8_t *row_class;   // [nrows]
+    const uint32_t *unit_off;   // units of the list's narrow rows before every entry
+    const uint32_t *part_off;   // partial sums of its narrow rows of several units before every entry
+    uint32_t *nbm;              // marked columns, kNarrowCols bits a narrow row (in the order of row_xi)
+    float2 *part;               // partial (sum, error) pairs, narrow_cols a unit
+    uint32_t narrow_cols;       // most columns of a job with narrow rows
     // symbolic output
     uint32_t *row_nnz;         // [nrows]
     // numeric output
@@ -153,6 +162,14 @@ void launch_heavy(const AccArgs &a, bool numeric, int grid, cudaStream_t s);
 // for those of at most kKeepBitsPerProduct (launch_heavy_bitmaps, rows.h).
 constexpr uint64_t kKeepBitsPerProduct = 32;
 constexpr uint64_t kKeepBitsMax = 512;
+// Narrow rows (narrow.cu): heavy rows of jobs with at most kNarrowCols distinct
+// columns and at least kNarrowProducts products a column.  8 warps' pairs of
+// 1024 columns are 64 KB, three CTAs an SM; the products a column pay for
+// adding the warps' pairs up and for the marks (32 words a row).
+constexpr int kNarrowCols = 1024;
+constexpr uint64_t kNarrowProducts = 16;
+constexpr uint64_t kNarrowSlice = 16384;  // products of a unit at least (2048 a warp)
+void launch_narrow(const AccArgs &a, bool numeric, int sm_count, cudaStream_t s);
 // numeric pass of single-run rows (their symbolic count is their product count)
 void launch_stream(const AccArgs &a, int grid, cudaStream_t s);
 int stream_blocks_per_sm();

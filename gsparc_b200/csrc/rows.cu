@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kScanThreads)
 __global__ void k_y_ranks(const uint64_t *__restrict__ ykeys, uint64_t ny, int kby, const BPrep *__restrict__ jobs,
                           int g, const uint32_t *__restrict__ bits, const uint32_t *__restrict__ wpre,
                           const uint64_t *__restrict__ cnts, uint32_t *__restrict__ rank, BatchJob *__restrict__ acc,
-                          const unsigned int *__restrict__ err) {
+                          const unsigned int *__restrict__ ydup, const unsigned int *__restrict__ err) {
     if (*err & kScanErr) return;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -165,6 +165,7 @@ __global__ void k_y_ranks(const uint64_t *__restrict__ ykeys, uint64_t ny, int k
     for (uint64_t j = t0; j < (uint64_t)g; j += stride) {
         BatchJob b;
         b.y_nfbits = jobs[j].y_nfbits;
+        b.ydup = ydup[j];
         b.cols_off = wpre[jobs[j].col_word0];
         b.ncols = (uint32_t)((j + 1 < (uint64_t)g ? wpre[jobs[j + 1].col_word0] : cnts[kCntCols]) - b.cols_off);
         acc[j] = b;
@@ -227,9 +228,10 @@ __global__ void __launch_bounds__(kScanThreads)
 
 // Row classes: single-run rows of jobs without repeated Y coordinates stream
 // (their output count is their product count), other rows with more than the
-// job's light limit of products are heavy, the rest with products are light.
+// job's light limit of products are heavy (narrow where the job has few
+// columns and the row many products for them), the rest with products are light.
 __global__ void __launch_bounds__(kScanThreads)
-    k_row_classes(const BPrep *__restrict__ jobs, const unsigned int *__restrict__ ydup,
+    k_row_classes(const BPrep *__restrict__ jobs, const BatchJob *__restrict__ acc,
                   const uint64_t *__restrict__ range, RowArrays r, uint64_t *__restrict__ cnts, ScanState st) {
     __shared__ ScanShared<4> sh;
     if (ld_acquire(st.err) & kScanErr) return;
@@ -240,7 +242,7 @@ __global__ void __launch_bounds__(kScanThreads)
     const uint64_t i0 = (uint64_t)tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
     uint8_t cl[kScanItems];
     uint64_t pr[kScanItems];
-    uint64_t x[4] = {0, 0, 0, 0};  // heavy and (above 32 bits) stream rows; light rows; light, stream products
+    uint64_t x[4] = {0, 0, 0, 0};  // heavy and (above 32 bits) stream rows; light and narrow rows; light, stream products
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) {
         const uint64_t i = i0 + q;
@@ -251,18 +253,24 @@ __global__ void __launch_bounds__(kScanThreads)
             const uint32_t k0 = r.row_k0[i], runs = r.row_k0[i + 1] - k0;
             if (i >= r0 && i < r1 && runs) {
                 const uint16_t j = r.row_job[i];
-                if (runs == 1 && !ydup[j]) {
+                if (runs == 1 && !acc[j].ydup) {
                     cl[q] = kRowStream;
                     r.row_xi[i] = r.mrun[k0];
                 } else {
                     cl[q] = pr[q] > jobs[j].light_max ? kRowHeavy : kRowLight;
+                    const uint32_t nc = acc[j].ncols;
+                    if (cl[q] == kRowHeavy && nc <= (uint32_t)kNarrowCols && pr[q] >= kNarrowProducts * nc) {
+                        cl[q] = kRowNarrow;
+                        if (cnts[kCntNarrowCols] < nc)
+                            atomicMax((unsigned long long *)&cnts[kCntNarrowCols], (unsigned long long)nc);
+                    }
                 }
             }
             r.row_prod[i] = pr[q];
             r.row_class[i] = cl[q];
             r.row_nnz[i] = cl[q] == kRowStream ? (uint32_t)pr[q] : 0u;
-            x[0] += (cl[q] == kRowHeavy) + ((uint64_t)(cl[q] == kRowStream) << 32);
-            x[1] += cl[q] == kRowLight;
+            x[0] += (cl[q] >= kRowHeavy) + ((uint64_t)(cl[q] == kRowStream) << 32);
+            x[1] += (cl[q] == kRowLight) + ((uint64_t)(cl[q] == kRowNarrow) << 32);
             x[2] += cl[q] == kRowLight ? pr[q] : 0;
             x[3] += cl[q] == kRowStream ? pr[q] : 0;
         }
@@ -271,18 +279,22 @@ __global__ void __launch_bounds__(kScanThreads)
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) {
         const uint32_t row = (uint32_t)(i0 + q);
-        if (cl[q] == kRowHeavy) {
+        if (cl[q] >= kRowHeavy) {
             r.H[(uint32_t)x[0]] = row;
             x[0] += 1;
+            if (cl[q] == kRowNarrow) {
+                r.row_xi[row] = (uint32_t)(x[1] >> 32);
+                x[1] += 1ull << 32;
+            }
         } else if (cl[q] == kRowStream) {
             r.SR[x[0] >> 32] = row;
             r.sprefix[x[0] >> 32] = x[3];
             x[0] += 1ull << 32;
             x[3] += pr[q];
         } else if (cl[q] == kRowLight) {
-            r.L[x[1]] = row;
-            r.lpre[x[1]] = x[2];
-            r.lbrk[x[1]] = (uint32_t)x[0] + (uint32_t)(x[0] >> 32);
+            r.L[(uint32_t)x[1]] = row;
+            r.lpre[(uint32_t)x[1]] = x[2];
+            r.lbrk[(uint32_t)x[1]] = (uint32_t)x[0] + (uint32_t)(x[0] >> 32);
             x[1] += 1;
             x[2] += pr[q];
         }
@@ -290,7 +302,8 @@ __global__ void __launch_bounds__(kScanThreads)
     if ((uint64_t)(tile + 1) * kScanTile >= nr && threadIdx.x == 0) {
         cnts[kCntHeavy] = (uint32_t)sh.through[0];
         cnts[kCntStream] = sh.through[0] >> 32;
-        cnts[kCntLight] = sh.through[1];
+        cnts[kCntLight] = (uint32_t)sh.through[1];
+        cnts[kCntNarrow] = sh.through[1] >> 32;
         r.sprefix[sh.through[0] >> 32] = sh.through[3];
     }
 }
@@ -397,7 +410,8 @@ __global__ void __launch_bounds__(kScanThreads)
         if (i0 + q < n) {
             const uint32_t row = r.H[i0 + q];
             const uint64_t span = (uint64_t)row_mx[row] - row_rb[row] + 1, prod = r.row_prod[row];
-            const uint32_t words = (uint32_t)(((span + 127) >> 7) << 2);
+            // narrow rows keep no bitmap here
+            const uint32_t words = r.row_class[row] == kRowHeavy ? (uint32_t)(((span + 127) >> 7) << 2) : 0u;
             wa[q] = span <= kKeepBitsMax * prod ? words : 0u;
             wd[q] = span <= kKeepBitsPerProduct * prod ? words : 0u;
             x[0] += wa[q];
@@ -447,9 +461,9 @@ void launch_col_table(const uint32_t *bits, uint64_t nwords, const BPrep *jobs, 
 
 void launch_y_ranks(const uint64_t *ykeys, uint64_t ny, int kby, const BPrep *jobs, int g, const uint32_t *bits,
                     const uint32_t *wpre, const uint64_t *cnts, uint32_t *rank, BatchJob *acc,
-                    const unsigned int *err, cudaStream_t s) {
+                    const unsigned int *ydup, const unsigned int *err, cudaStream_t s) {
     k_y_ranks<<<grid_for(std::max<uint64_t>(ny, (uint64_t)g)), kThreads, 0, s>>>(ykeys, ny, kby, jobs, g, bits, wpre,
-                                                                                cnts, rank, acc, err);
+                                                                                cnts, rank, acc, ydup, err);
     launched();
 }
 
@@ -460,10 +474,10 @@ void launch_x_rows(const uint64_t *xkeys, uint64_t nx, int kbx, const BPrep *job
     launched();
 }
 
-void launch_row_classes(uint64_t nx, const BPrep *jobs, const unsigned int *ydup, const uint64_t *range,
+void launch_row_classes(uint64_t nx, const BPrep *jobs, const BatchJob *acc, const uint64_t *range,
                         const RowArrays &r, uint64_t *cnts, const ScanState &st, cudaStream_t s) {
     if (nx == 0) return;
-    k_row_classes<<<(unsigned)scan_tiles(nx), kScanThreads, 0, s>>>(jobs, ydup, range, r, cnts, st);
+    k_row_classes<<<(unsigned)scan_tiles(nx), kScanThreads, 0, s>>>(jobs, acc, range, r, cnts, st);
     launched();
 }
 

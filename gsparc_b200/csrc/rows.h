@@ -28,10 +28,12 @@ enum {
     kCntRange = 9,    // 9..11 shard row range and products
     kCntBmAll = 12,   // words of every kept bitmap
     kCntBmDense = 13, // words of the dense rows' kept bitmaps
+    kCntNarrow = 14,     // narrow rows among the heavy ones
+    kCntNarrowCols = 15, // most columns of a job with narrow rows
     kCnts = 16
 };
 
-constexpr uint8_t kRowNone = 0, kRowLight = 1, kRowStream = 2, kRowHeavy = 3;
+constexpr uint8_t kRowNone = 0, kRowLight = 1, kRowStream = 2, kRowHeavy = 3, kRowNarrow = 4;  // narrow: heavy, over few columns
 
 // Sorted Y keys -> run table (run_key, run_start with the closing entry, count
 // in cnts), ydup per job; marks every entry's free index in the presence bits
@@ -46,7 +48,7 @@ void launch_col_table(const uint32_t *bits, uint64_t nwords, const BPrep *jobs, 
 // Column rank of every Y entry inside its job, and the jobs' column ranges.
 void launch_y_ranks(const uint64_t *ykeys, uint64_t ny, int kby, const BPrep *jobs, int g, const uint32_t *bits,
                     const uint32_t *wpre, const uint64_t *cnts, uint32_t *rank, BatchJob *acc,
-                    const unsigned int *err, cudaStream_t s);
+                    const unsigned int *ydup, const unsigned int *err, cudaStream_t s);
 
 struct RowArrays {
     uint64_t *xprefix;   // [nx + 1] matched products before every X nonzero
@@ -60,7 +62,7 @@ struct RowArrays {
     uint64_t *row_prod;  // [nrows]
     uint8_t *row_class;  // [nrows]
     uint32_t *row_nnz;   // [nrows] stream rows: their products; 0 otherwise
-    uint32_t *row_xi;    // [nrows] stream rows: their matched X nonzero
+    uint32_t *row_xi;    // [nrows] stream rows: their matched X nonzero; narrow rows: their number
     uint32_t *H, *SR, *L;  // heavy, stream and light rows, in row order
     uint64_t *sprefix;   // [stream + 1] products before every stream row
     uint64_t *lpre;      // [light] products of the light rows before each one
@@ -71,7 +73,7 @@ struct RowArrays {
 void launch_x_rows(const uint64_t *xkeys, uint64_t nx, int kbx, const BPrep *jobs, const uint32_t *cnt,
                    const uint8_t *row_flag, const RowArrays &r, uint64_t *cnts, const ScanState &st, cudaStream_t s);
 // Row classes, their lists and product prefixes (rows outside `range` get no class).
-void launch_row_classes(uint64_t nx, const BPrep *jobs, const unsigned int *ydup, const uint64_t *range,
+void launch_row_classes(uint64_t nx, const BPrep *jobs, const BatchJob *acc, const uint64_t *range,
                         const RowArrays &r, uint64_t *cnts, const ScanState &st, cudaStream_t s);
 // Light units of at most bin + light_max products.
 void launch_light_units(uint64_t nx, uint64_t bin, const RowArrays &r, uint64_t *cnts, const ScanState &st,
@@ -82,5 +84,10 @@ void launch_light_units(uint64_t nx, uint64_t bin, const RowArrays &r, uint64_t 
 void launch_heavy_bitmaps(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, const uint32_t *yrank,
                           const RowArrays &r, uint32_t *row_rb, uint32_t *row_mx, uint32_t *w_all, uint32_t *w_dense,
                           uint64_t *off_all, uint64_t *off_dense, uint64_t *cnts, const ScanState &st, cudaStream_t s);
+
+// unit_off[0..n] and part_off[0..n) of a heavy list (narrow.cu), units of about
+// `slice` products.
+void launch_narrow_units(const uint32_t *list, uint32_t n, const uint8_t *row_class, const uint64_t *row_prod,
+                         uint64_t slice, uint32_t *unit_off, uint32_t *part_off, const ScanState &st, cudaStream_t s);
 
 }  // namespace gs

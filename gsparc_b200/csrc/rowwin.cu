@@ -42,6 +42,7 @@
 // column, so gaps are skipped.
 #include "blockops.cuh"
 #include "kernels.cuh"
+#include "rows.h"
 
 namespace gs {
 
@@ -398,6 +399,7 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
     __shared__ uint32_t s_cut;
     __shared__ uint32_t s_next;  // kept bitmaps: the smallest rank past the window (atomicMin)
     __shared__ RowConst s_rc;
+    __shared__ uint32_t s_rows;  // rows of the list before its narrow rows
 
     const int tid = threadIdx.x;
     // outputs per window: the compiled capacity, or a smaller tile chosen at run time
@@ -406,13 +408,25 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
     for (int i = tid; i < NWK; i += T) bits[i] = 0;
     if (NUMERIC)
         for (int i = tid; i < CAP; i += T) hi[i] = lo[i] = 0.f;
+    if (tid == 0) {
+        uint32_t lo_r = a.row_class ? 0u : a.nunits, hi_r = a.nunits;
+        while (lo_r < hi_r) {
+            const uint32_t mid = (lo_r + hi_r) >> 1;
+            if (a.row_class[a.units[mid]] != kRowNarrow)
+                lo_r = mid + 1;
+            else
+                hi_r = mid;
+        }
+        s_rows = hi_r;
+    }
     __syncthreads();
+    const uint32_t nrows = s_rows;
 
     for (;;) {
         if (tid == 0) s_unit = atomicAdd(a.work_counter, 1u);
         __syncthreads();
         const uint32_t u = s_unit;
-        if (u >= a.nunits) break;
+        if (u >= nrows) break;
         const uint32_t row = a.units[u];
         const uint32_t xs = a.row_start[row], xe = a.row_start[row + 1];
         // words of the row's kept column bitmap (0: none, the windows mark their columns)
