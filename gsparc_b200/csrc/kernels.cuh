@@ -24,17 +24,17 @@ void launch_linearize(const LinParams &p, uint64_t nnz, const uint64_t *idx, con
                       uint64_t *keys, float *val_out, unsigned int *err, cudaStream_t s);
 
 // ---- sort (CUB radix sort; reference: include/gsparc/sort.cuh:90-108) ----
-// Sorts (keys, vals) by bits [0, nbits).  keys/vals are double buffers: on
+// Sorts (keys, vals) by bits [begin, nbits).  keys/vals are double buffers: on
 // return *which tells which of the two holds the result (0 or 1).
 void sort_pairs(Arena &a, uint64_t n, uint64_t *keys0, uint64_t *keys1, float *vals0, float *vals1,
-                int nbits, int *which, cudaStream_t s);
+                int nbits, int *which, cudaStream_t s, int begin = 0);
 void sort_keys(Arena &a, uint64_t n, uint64_t *keys0, uint64_t *keys1, int nbits, int *which,
                cudaStream_t s);
 // This library's own stable onesweep radix sort of the same pairs (radix.cu),
 // 8 bits per pass; same double-buffer contract as sort_pairs.  A look-back
 // wait that runs out sets bit 8 of *err (the caller's device error word).
 void own_sort_pairs(Arena &a, uint64_t n, uint64_t *keys0, uint64_t *keys1, float *vals0, float *vals1,
-                    int nbits, int *which, unsigned int *err, cudaStream_t s);
+                    int nbits, int *which, unsigned int *err, cudaStream_t s, int begin = 0);
 
 // ---- Y preparation ----
 // From sorted Y keys (c << nfbits | f): per-entry column rank among the

@@ -247,16 +247,16 @@ void launch_linearize(const LinParams &p, uint64_t nnz, const uint64_t *idx, con
 }
 
 void sort_pairs(Arena &a, uint64_t n, uint64_t *keys0, uint64_t *keys1, float *vals0, float *vals1,
-                int nbits, int *which, cudaStream_t s) {
+                int nbits, int *which, cudaStream_t s, int begin) {
     *which = 0;
-    if (n <= 1 || nbits <= 0) return;
+    if (n <= 1 || nbits <= begin) return;
     GS_REQUIRE(n < (1ull << 31), GSPARC_EUNSUPPORTED, "sort of more than 2^31 entries");
     cub::DoubleBuffer<uint64_t> kb(keys0, keys1);
     cub::DoubleBuffer<float> vb(vals0, vals1);
     size_t tmp = 0;
-    GS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, kb, vb, (int)n, 0, nbits, s));
+    GS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, kb, vb, (int)n, begin, nbits, s));
     DBuf<uint8_t> t(a, tmp, s);
-    GS_CUDA(cub::DeviceRadixSort::SortPairs(t.get(), tmp, kb, vb, (int)n, 0, nbits, s));
+    GS_CUDA(cub::DeviceRadixSort::SortPairs(t.get(), tmp, kb, vb, (int)n, begin, nbits, s));
     *which = kb.selector;
 }
 

@@ -3,7 +3,7 @@
 // include/gsparc/sort.cuh:90-108).  Selected per context by
 // gsparc_ctx_set_sort; CUB stays the default.
 //
-// Onesweep form: 8 bits per pass over [0, nbits), the last pass masked to the
+// Onesweep form: 8 bits per pass over [begin, nbits), the last pass masked to the
 // bits below nbits.
 //   1. k_os_hist reads every key once and counts the digits of all passes
 //      (shared-memory counts per block, lanes of one digit aggregated by
@@ -88,8 +88,8 @@ __device__ __forceinline__ uint32_t block_excl_scan256(uint32_t x, uint32_t *s_w
 }
 
 // Digit counts of every pass: gh[p * 256 + d].
-__global__ void __launch_bounds__(kOsThreads) k_os_hist(const uint64_t *__restrict__ keys, uint64_t n, int nbits,
-                                                        int npass, uint32_t *__restrict__ gh) {
+__global__ void __launch_bounds__(kOsThreads) k_os_hist(const uint64_t *__restrict__ keys, uint64_t n, int begin,
+                                                        int nbits, int npass, uint32_t *__restrict__ gh) {
     __shared__ uint32_t h[kMaxPass * 256];
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t lt = (1u << lane) - 1u;
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(kOsThreads) k_os_hist(const uint64_t *__restri
         const bool ok = i < n;
         const uint64_t k = ok ? keys[i] : 0ull;
         for (int p = 0; p < npass; ++p) {
-            const int shift = 8 * p;
+            const int shift = begin + 8 * p;
             const uint32_t d = ok ? digit_of(k, shift, pass_mask(nbits, shift)) : 256u + (uint32_t)lane;
             const uint32_t peers = __match_any_sync(FULL, d);
             if (ok && (peers & lt) == 0) atomicAdd(&h[p * 256 + d], (uint32_t)__popc(peers));
@@ -230,22 +230,22 @@ constexpr size_t kPassSmem = (size_t)kTile * (8 + 4) + 4 * (kOsWarps * 256 + 256
 }  // namespace
 
 void own_sort_pairs(Arena &a, uint64_t n, uint64_t *keys0, uint64_t *keys1, float *vals0, float *vals1, int nbits,
-                    int *which, unsigned int *err, cudaStream_t s) {
+                    int *which, unsigned int *err, cudaStream_t s, int begin) {
     *which = 0;
-    if (n <= 1 || nbits <= 0) return;
+    if (n <= 1 || nbits <= begin) return;
     GS_REQUIRE(n < (1ull << 30), GSPARC_EUNSUPPORTED, "own radix sort of 2^30 entries or more");
     GS_CUDA(cudaFuncSetAttribute(k_os_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPassSmem));
-    const int npass = (nbits + 7) / 8;
+    const int npass = (nbits - begin + 7) / 8;
     const uint32_t ntiles = (uint32_t)((n + kTile - 1) / kTile);
     DBuf<uint32_t> gh(a, (uint64_t)npass * 256, s), status(a, (uint64_t)ntiles * 256 + 1, s);
     GS_CUDA(cudaMemsetAsync(gh.get(), 0, 4ull * npass * 256, s));
     const uint64_t hblocks = std::min<uint64_t>((n + kOsThreads - 1) / kOsThreads, 148ull * 8);
-    k_os_hist<<<(unsigned)hblocks, kOsThreads, 0, s>>>(keys0, n, nbits, npass, gh);
+    k_os_hist<<<(unsigned)hblocks, kOsThreads, 0, s>>>(keys0, n, begin, nbits, npass, gh);
     count_launch();
     uint64_t *kin = keys0, *kout = keys1;
     float *vin = vals0, *vout = vals1;
     for (int p = 0; p < npass; ++p) {
-        const int shift = 8 * p;
+        const int shift = begin + 8 * p;
         GS_CUDA(cudaMemsetAsync(status.get(), 0, 4ull * ntiles * 256 + 4, s));
         k_os_pass<<<ntiles, kOsThreads, kPassSmem, s>>>(kin, vin, n, shift, pass_mask(nbits, shift), ntiles,
                                                         gh.get() + 256 * p, status, err, kout, vout);

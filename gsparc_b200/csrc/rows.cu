@@ -40,13 +40,14 @@ __device__ __forceinline__ uint64_t low_mask(int b) { return b >= 64 ? ~0ull : (
 __global__ void __launch_bounds__(kScanThreads)
     k_y_runs(const uint64_t *__restrict__ ykeys, uint64_t ny, int kby, const BPrep *__restrict__ jobs,
              uint64_t *__restrict__ run_key, uint32_t *__restrict__ run_start, uint64_t *__restrict__ cnts,
-             unsigned int *__restrict__ ydup, uint32_t *__restrict__ bits, uint64_t *__restrict__ yfk, ScanState st) {
+             unsigned int *__restrict__ ydup, uint32_t *__restrict__ bits, uint64_t *__restrict__ yfk,
+             uint2 *__restrict__ ctab, ScanState st) {
     __shared__ ScanShared<1> sh;
     const uint32_t tile = next_tile(st, sh);
     const uint64_t i0 = (uint64_t)tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
     const uint64_t km = low_mask(kby);
     uint64_t rk[kScanItems];
-    uint32_t flags = 0;
+    uint32_t flags = 0, first = 0;  // bit q: a run starts there; it is the first of its table word
     uint64_t pk = i0 > 0 && i0 < ny ? ykeys[i0 - 1] : 0;
     uint64_t pj = ~0ull, prk = 0;
     if (i0 > 0 && i0 < ny) {
@@ -65,7 +66,10 @@ __global__ void __launch_bounds__(kScanThreads)
             const BPrep b = jobs[j];
             const uint64_t loc = key & km;
             rk[q] = shr(loc, b.y_nfbits);
-            if (j != pj || rk[q] != prk) flags |= 1u << q;
+            if (j != pj || rk[q] != prk) {
+                flags |= 1u << q;
+                if (j != pj || (rk[q] >> 5) != (prk >> 5)) first |= 1u << q;
+            }
             if (i > 0 && pk == key) atomicOr(&ydup[j], 1u);
             pk = key;
             pj = j;
@@ -94,6 +98,14 @@ __global__ void __launch_bounds__(kScanThreads)
         if (flags >> q & 1u) {
             run_key[x[0]] = rk[q];
             run_start[x[0]] = (uint32_t)(i0 + q);
+            if (ctab) {
+                const BPrep b = jobs[shr(rk[q], kby)];
+                // masked: an out-of-range index (its job fails) stays in its job's words
+                const uint64_t c = rk[q] & km & low_mask(b.x_ncbits);
+                uint2 *t = ctab + b.con_word0 + (c >> 5);
+                atomicOr(&t->x, 1u << (c & 31));
+                if (first >> q & 1u) t->y = (uint32_t)x[0];
+            }
             ++x[0];
         }
     if ((uint64_t)(tile + 1) * kScanTile >= ny && threadIdx.x == 0) {
@@ -445,10 +457,10 @@ void launched() {
 
 void launch_y_runs(const uint64_t *ykeys, uint64_t ny, int kby, const BPrep *jobs, uint64_t *run_key,
                    uint32_t *run_start, uint64_t *cnts, unsigned int *ydup, uint32_t *bits, uint64_t *yfk,
-                   const ScanState &st, cudaStream_t s) {
+                   uint2 *ctab, const ScanState &st, cudaStream_t s) {
     if (ny == 0) return;
     k_y_runs<<<(unsigned)scan_tiles(ny), kScanThreads, 0, s>>>(ykeys, ny, kby, jobs, run_key, run_start, cnts, ydup,
-                                                               bits, yfk, st);
+                                                               bits, yfk, ctab, st);
     launched();
 }
 

@@ -13,6 +13,7 @@ struct BPrep {
     int y_nfbits;
     uint64_t light_max;  // rows with more products go to the windowed accumulator
     uint64_t col_word0;  // first word of the job's Y free indices in the presence bits
+    uint64_t con_word0;  // first word of the job's contract keys in the run lookup table
 };
 
 // Device counters of a group.
@@ -37,10 +38,12 @@ constexpr uint8_t kRowNone = 0, kRowLight = 1, kRowStream = 2, kRowHeavy = 3, kR
 
 // Sorted Y keys -> run table (run_key, run_start with the closing entry, count
 // in cnts), ydup per job; marks every entry's free index in the presence bits
-// (bits null: writes the prefixed free index to yfk instead).
+// (bits null: writes the prefixed free index to yfk instead).  With ctab (zero
+// at entry), also the run lookup table: for every 32 contract keys of a job
+// the keys that have a run (word 0) and the first of these runs (word 1).
 void launch_y_runs(const uint64_t *ykeys, uint64_t ny, int kby, const BPrep *jobs, uint64_t *run_key,
                    uint32_t *run_start, uint64_t *cnts, unsigned int *ydup, uint32_t *bits, uint64_t *yfk,
-                   const ScanState &st, cudaStream_t s);
+                   uint2 *ctab, const ScanState &st, cudaStream_t s);
 // Presence bits -> distinct free indices of every job (cols, ascending) and
 // the number of distinct ones before every word (wpre).
 void launch_col_table(const uint32_t *bits, uint64_t nwords, const BPrep *jobs, int g, uint32_t *wpre, uint64_t *cols,

@@ -70,3 +70,19 @@ def test_shards(ctx, nshards):
     parts = [gb.sptc(ctx, dx, dy, [1], [0], shard=k, nshards=nshards) for k in range(nshards)]
     assert np.array_equal(np.concatenate([p.keys for p in parts]), z.keys)
     value_bar.max_rel_err(np.concatenate([p.vals for p in parts]), z.vals)
+
+
+@pytest.mark.parametrize("space", [2, 31, 32, 33, 5000, 1 << 28])  # 2^28: runs found by search
+def test_contract_space(ctx, space):
+    rng = np.random.default_rng(space)
+    used = np.unique(np.concatenate([rng.integers(0, space, 900), [0, space - 1]]))
+    x = np.stack([rng.integers(0, 500, 6000), rng.choice(used, 6000)]).astype(np.uint64)
+    y = np.stack([rng.choice(used[::2], 3000), rng.integers(0, 400, 3000)]).astype(np.uint64)
+    X = gb.CooTensor([500, space], x, rng.standard_normal(6000).astype(np.float32))
+    Y = gb.CooTensor([space, 400], y, rng.standard_normal(3000).astype(np.float32))
+    for sort in (0, 1):
+        ctx.set_sort(sort)
+        try:
+            _same(gb.SpTC(X, Y, [1], [0], ctx=ctx), ob.sptc(X, Y, [1], [0]))
+        finally:
+            ctx.set_sort(0)
