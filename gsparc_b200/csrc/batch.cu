@@ -273,42 +273,23 @@ __global__ void k_heavy_sizes(const uint32_t *__restrict__ H, uint64_t nh, const
     }
 }
 
-// Light units first-row search: light units starting before row r.
-__device__ __forceinline__ uint64_t light_before(const uint32_t *units, uint64_t nu, uint32_t r) {
-    uint64_t lo = 0, hi = nu;
-    while (lo < hi) {
-        const uint64_t mid = (lo + hi) >> 1;
-        if (units[2 * mid] < r)
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    return lo;
-}
-
-// The three unit lists of a group, all in row order: light units (row
-// pairs), heavy rows and single-run (stream) rows.
+// The three row lists of a group, all in row order: light, heavy and
+// single-run (stream) rows.
 struct UnitLists {
-    const uint32_t *units;
-    uint64_t nu;
+    const uint32_t *L;
+    uint64_t nl;
     const uint32_t *H;
     uint64_t nh;
     const uint32_t *SR;
     uint64_t ns;
-    __device__ uint64_t size() const { return nu + nh + ns; }
-    // first row of unit k of the concatenation light | heavy | stream
-    __device__ uint32_t row(uint64_t k, uint32_t *last) const {
-        if (k < nu) {
-            *last = units[2 * k + 1];
-            return units[2 * k];
-        }
-        const uint32_t r = k < nu + nh ? H[k - nu] : SR[k - nu - nh];
-        *last = r + 1;
-        return r;
+    __device__ uint64_t size() const { return nl + nh + ns; }
+    // row k of the concatenation light | heavy | stream
+    __device__ uint32_t row(uint64_t k) const {
+        return k < nl ? L[k] : (k < nl + nh ? H[k - nl] : SR[k - nl - nh]);
     }
-    // units of all three lists that start before row r
+    // rows of all three lists before row r
     __device__ uint64_t before(uint32_t r) const {
-        return light_before(units, nu, r) + lower_bound_dev<uint32_t>(H, 0, nh, r) +
+        return lower_bound_dev<uint32_t>(L, 0, nl, r) + lower_bound_dev<uint32_t>(H, 0, nh, r) +
                lower_bound_dev<uint32_t>(SR, 0, ns, r);
     }
 };
@@ -330,9 +311,8 @@ __global__ void k_after_counts(UnitLists u, const uint64_t *__restrict__ row_off
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     uint64_t m = 0;
     for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < u.size(); k += stride) {
-        uint32_t r1;
-        const uint32_t r0 = u.row(k, &r1);
-        const uint64_t v = row_off[r1] - row_off[r0];
+        const uint32_t r = u.row(k);
+        const uint64_t v = row_off[r + 1] - row_off[r];
         m = v > m ? v : m;
     }
 #pragma unroll
@@ -349,8 +329,7 @@ __global__ void k_merge_starts(UnitLists u, const uint64_t *__restrict__ row_off
                                uint64_t *__restrict__ uoff) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < u.size(); k += stride) {
-        uint32_t r1;
-        const uint32_t r = u.row(k, &r1);
+        const uint32_t r = u.row(k);
         const uint64_t p = u.before(r);
         urow[p] = r;
         uoff[p] = row_off[r];
@@ -359,7 +338,7 @@ __global__ void k_merge_starts(UnitLists u, const uint64_t *__restrict__ row_off
 
 // Chunk k starts at the first unit whose output starts at or after
 // target[k] (target[0] = 0, increasing).  info[5k..5k+4] = first row, first
-// output, first light unit, first heavy row (row-ordered index), first stream
+// output, first light row, first heavy row (row-ordered index), first stream
 // row of chunk k; entry K closes the last chunk.
 constexpr int kChunkInfo = 5;
 __global__ void k_chunk_bounds(const uint32_t *__restrict__ urow, const uint64_t *__restrict__ uoff, uint64_t M,
@@ -372,7 +351,7 @@ __global__ void k_chunk_bounds(const uint32_t *__restrict__ urow, const uint64_t
         uint64_t *o = info + kChunkInfo * k;
         o[0] = row;
         o[1] = b < M ? uoff[b] : ntot;
-        o[2] = light_before(u.units, u.nu, row);
+        o[2] = lower_bound_dev<uint32_t>(u.L, 0, u.nl, row);
         o[3] = lower_bound_dev<uint32_t>(u.H, 0, u.nh, row);
         o[4] = lower_bound_dev<uint32_t>(u.SR, 0, u.ns, row);
     }
@@ -452,8 +431,8 @@ struct GroupPlan {
     DBuf<float> xperm, yperm, xvals, yvals;
     DBuf<uint64_t> ykeys;  // sorted Y keys (the single-run-row copy reads y_f from them)
     DBuf<BatchJob> d_acc;
-    DBuf<uint32_t> rank, pos, cnt, mpre, mrun, row_start, units, H, H2, SR, row_xi, cursor, pend;
-    DBuf<uint64_t> cols, xprefix, row_xf, sprefix, row_off;
+    DBuf<uint32_t> rank, pos, cnt, mpre, mrun, row_start, L, ustart, lk0, lrun, lrow, H, H2, SR, row_xi, cursor, pend;
+    DBuf<uint64_t> cols, xprefix, row_xf, sprefix, row_off, lpre, loff;
     DBuf<uint16_t> row_job;
     DBuf<uint32_t> Hc;         // heavy rows grouped by chunk (several chunks only)
     DBuf<uint32_t> hbm, row_rb, row_bmw;  // heavy rows' kept column bitmaps (may be empty)
@@ -585,7 +564,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     uint32_t *const ybits = col_bits ? flags_x + 6 * zf_x : nullptr;
     // the scans' sums (one buffer: the scans follow one another on the stream)
     DBuf<uint64_t> scan_vals(A, std::max({scan_value_words<1>(ny), col_bits ? scan_value_words<1>(col_words) : 0,
-                                          scan_value_words<4>(nx)}), s);
+                                          scan_value_words<kMaxScanSums>(nx)}), s);
     auto scan_state = [&](uint32_t *flags) { return ScanState{flags, scan_vals.get(), ctx->d_flag}; };
     h2d(d_lx.get(), lx.data(), g, s);
     h2d(d_ly.get(), ly.data(), g, s);
@@ -684,7 +663,8 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     DBuf<uint32_t> row_start(A, nx + 1, s);
     DBuf<uint64_t> row_xf(A, nxb, s), row_prod(A, nxb, s);
     DBuf<uint16_t> row_job(A, nxb, s);
-    DBuf<uint32_t> H(A, nxb, s), units(A, 2 * nxb, s);
+    DBuf<uint32_t> H(A, nxb, s), L(A, nxb, s), ustart(A, nx + 1, s), lk0(A, nx + 1, s), lrun(A, nxb, s), lrow(A, nxb, s);
+    DBuf<uint64_t> lpre(A, nx + 1, s), loff(A, nxb, s);
     DBuf<uint32_t> mpre(A, nx + 1, s), mrun(A, nxb, s), row_xi(A, nxb, s), SR(A, nxb, s);
     DBuf<uint64_t> sprefix(A, nx + 1, s);
     DBuf<uint32_t> row_nnz(A, nxb, s);
@@ -704,8 +684,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     if (nx) {
         DBuf<uint8_t> rflag(A, nx, s);
         row_class.reset(A, nx, s);
-        DBuf<uint32_t> mrow(A, nx, s), row_k0(A, nx + 1, s), L(A, nx, s), lbrk(A, nx, s);
-        DBuf<uint64_t> lpre(A, nx, s);
+        DBuf<uint32_t> mrow(A, nx, s), row_k0(A, nx + 1, s);
         k_bmatch<<<grid_for(nx), kThreads, 0, s>>>(xkeys, nx, kbx, kby, d_bp, run_key, run_start, cnts + kCntRuns,
                                                     ctab, pos, cnt, rflag);
         count_launch();
@@ -728,8 +707,11 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         ra.L = L;
         ra.sprefix = sprefix;
         ra.lpre = lpre;
-        ra.lbrk = lbrk;
-        ra.units = units;
+        ra.lk0 = lk0;
+        ra.ustart = ustart;
+        ra.lrun = lrun;
+        ra.lrow = lrow;
+        ra.loff = loff;
         launch_x_rows(xkeys, nx, kbx, d_bp, cnt, rflag, ra, cnts, scan_state(flags_x), s);
         const uint64_t *range = nullptr;
         if (nshards > 1) {
@@ -742,13 +724,16 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         launch_row_classes(nx, d_bp, d_acc, range, ra, cnts, scan_state(flags_x + zf_x), s);
         mark(3);
         launch_light_units(nx, light_bin, ra, cnts, scan_state(flags_x + 2 * zf_x), s);
+        DBuf<uint32_t> row_mx;
         if (keep_bm) {
-            DBuf<uint32_t> row_mx(A, nx, s);
+            row_mx.reset(A, nx, s);
             GS_CUDA(cudaMemsetAsync(row_rb.get(), 0xff, 4 * nx, s));
             GS_CUDA(cudaMemsetAsync(row_mx.get(), 0, 4 * nx, s));
-            launch_heavy_bitmaps(nx, pos, cnt, rank, ra, row_rb, row_mx, bm_w_all, bm_w_dense, bm_off_all,
-                                 bm_off_dense, cnts, scan_state(flags_x + 3 * zf_x), s);
         }
+        launch_matched_runs(nx, pos, cnt, rank, ra, row_rb, row_mx, cnts, ctx->d_flag, s);
+        if (keep_bm)
+            launch_heavy_bitmaps(nx, ra, row_rb, row_mx, bm_w_all, bm_w_dense, bm_off_all, bm_off_dense, cnts,
+                                 scan_state(flags_x + 3 * zf_x), s);
     } else {
         GS_CUDA(cudaMemsetAsync(xprefix.get(), 0, 8, s));
         GS_CUDA(cudaMemsetAsync(mpre.get(), 0, 4, s));
@@ -766,8 +751,8 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     GS_CUDA(cudaStreamSynchronize(s));
     GS_REQUIRE(!(herr & kScanErr), GSPARC_EINTERNAL, "a prefix sum's or the radix sort's look-back gave up");
     const uint64_t bm_words_all = hc_cnt[kCntBmAll], bm_words_dense = hc_cnt[kCntBmDense];
-    const uint64_t nrows = hc_cnt[kCntRows], nh = hc_cnt[kCntHeavy], nu = hc_cnt[kCntUnits],
-                   nsr = hc_cnt[kCntStream];
+    const uint64_t nrows = hc_cnt[kCntRows], nh = hc_cnt[kCntHeavy], nl = hc_cnt[kCntLight],
+                   nu = hc_cnt[kCntUnits], nsr = hc_cnt[kCntStream];
     if (nshards > 1) ir = hc_cnt[kCntRange + 2];  // the shard's products
     bst.ir_nnz += ir;
     bst.rows += nrows;
@@ -817,6 +802,29 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     aa.mpre = mpre;
     aa.mrun = mrun;
     aa.light_cap = (uint32_t)light_cap;
+    aa.light_cols = hc_cnt[kCntCols];
+    aa.ustart = ustart;
+    aa.lk0 = lk0;
+    aa.lrun = lrun;
+    aa.lrow = lrow;
+    aa.lpre = lpre;
+    aa.loff = loff;
+    // Light rows are merged once: the pass that counts their outputs writes them
+    // to scratch, 12 B a product, which the chunks copy from; twice (the second
+    // time in place) where that does not fit an eighth of the memory left, and
+    // for plans, whose values change.
+    const uint64_t light_prod = hc_cnt[kCntLightProd];
+    const bool light_once = !keep && nu && light_prod * 12 <= A.available() / 8;
+    DBuf<uint64_t> lout_keys, lpos;
+    DBuf<float> lout_vals;
+    if (light_once) {
+        lout_keys.reset(A, light_prod, s);
+        lout_vals.reset(A, light_prod, s);
+        lpos.reset(A, nl, s);
+        aa.lpos = lpos;
+        aa.lout_keys = lout_keys;
+        aa.lout_vals = lout_vals;
+    }
     aa.xval = xvals;
     aa.yrank = rank;
     aa.yval = yvals;
@@ -883,10 +891,14 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     const int gs_grid = std::max(1, ctx->sm_count * stream_blocks_per_sm());
     {
         AccArgs b = aa;
-        b.units = units;
+        b.units = L;
         b.nunits = (uint32_t)nu;
+        b.l0 = 0;
+        b.l1 = (uint32_t)nl;
         GS_CUDA(cudaMemsetAsync(ctx->d_flag + 1, 0, 4, s));
-        launch_light(b, false, (int)std::min<uint64_t>(gl, std::max<uint64_t>(1, nu)), s);
+        b.out_cap = light_prod;
+        launch_light(b, light_once ? kLightValues : kLightCount,
+                     (int)std::min<uint64_t>(gl, std::max<uint64_t>(1, nu)), s);
         b.units = Hs;
         b.nunits = (uint32_t)nh;
         if (nh > nnarrow) {
@@ -900,8 +912,8 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     }
     exclusive_scan_u32_to_u64(A, row_nnz, row_off, nrows, s);
     DBuf<JobOut> d_jo(A, g + 1, s);
-    const UnitLists ul{units, nu, H, nh, SR, nsr};
-    k_after_counts<<<grid_for(std::max<uint64_t>(nu + nh + nsr, (uint64_t)g + 1)), kThreads, 0, s>>>(
+    const UnitLists ul{L, nl, H, nh, SR, nsr};
+    k_after_counts<<<grid_for(std::max<uint64_t>(nl + nh + nsr, (uint64_t)g + 1)), kThreads, 0, s>>>(
         ul, row_off, row_job, nrows, xprefix, d_xoffs, g, d_jo, cnts + kCntMaxUnit);
     count_launch();
     GS_CUDA(cudaGetLastError());
@@ -944,7 +956,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     if (max_chunk_nnz) cap = std::min(cap, max_chunk_nnz);
     cap = std::max<uint64_t>(cap, 1);
     struct Chunk {
-        uint64_t lu0, lu1;  // light units [lu0, lu1)
+        uint64_t lu0, lu1;  // light rows [lu0, lu1)
         uint64_t h0, h1;    // heavy rows [h0, h1) of the chunk-grouped heavy list
         uint64_t s0, s1;    // stream rows [s0, s1)
         uint64_t first, n;
@@ -956,7 +968,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     // kFirstCutProducts, 2x that, 4x that, ... products.
     const bool progressive = done_fn && g > 1 && ntot > 0;
     if (ntot <= cap && !progressive) {
-        if (ntot || nu || nh || nsr) chunks.push_back({0, nu, 0, nh, 0, nsr, 0, ntot});
+        if (ntot || nl || nh || nsr) chunks.push_back({0, nl, 0, nh, 0, nsr, 0, ntot});
     } else {
         uint64_t C = std::max(cap > max_unit ? cap - max_unit : 1, std::max<uint64_t>(max_unit, 1));
         C = std::max<uint64_t>(C, (ntot + (1ull << 20) - 1) >> 20);  // at most 2^20 uniform chunks
@@ -980,7 +992,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         }
         target.push_back(ntot);
         const uint64_t K = target.size() - 1;
-        const uint64_t M = nu + nh + nsr;
+        const uint64_t M = nl + nh + nsr;
         DBuf<uint32_t> urow(A, M, s);
         DBuf<uint64_t> uoff(A, M, s);
         k_merge_starts<<<grid_for(M), kThreads, 0, s>>>(ul, row_off, urow, uoff);
@@ -1047,8 +1059,14 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         keep->cnt = std::move(cnt);
         keep->mpre = std::move(mpre);
         keep->mrun = std::move(mrun);
+        keep->ustart = std::move(ustart);
+        keep->lk0 = std::move(lk0);
+        keep->lrun = std::move(lrun);
+        keep->lrow = std::move(lrow);
+        keep->lpre = std::move(lpre);
+        keep->loff = std::move(loff);
         keep->row_start = std::move(row_start);
-        keep->units = std::move(units);
+        keep->L = std::move(L);
         keep->H = std::move(H);
         keep->H2 = std::move(H2);
         keep->SR = std::move(SR);
@@ -1166,11 +1184,17 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         b.out_keys = out_k[bi];
         b.out_vals = out_v[bi];
         b.out_cap = c.n;
-        b.units = units.get() + 2 * c.lu0;
-        b.nunits = (uint32_t)(c.lu1 - c.lu0);
+        b.units = L;
+        b.nunits = (uint32_t)nu;
+        b.l0 = (uint32_t)c.lu0;
+        b.l1 = (uint32_t)c.lu1;
         GS_CUDA(cudaMemsetAsync(counter, 0, 4, sc));
         GS_CUDA(cudaEventRecord(kev[2 * ci], sc));
-        launch_light(b, true, (int)std::min<uint64_t>(gl, std::max<uint64_t>(1, b.nunits)), sc);
+        if (light_once) {
+            launch_light_copy(b, ctx->sm_count, sc);
+        } else {
+            launch_light(b, kLightFinal, (int)std::min<uint64_t>(gl, std::max<uint64_t>(1, nu)), sc);
+        }
         b.units = Hchunk + c.h0;
         b.nunits = (uint32_t)(c.h1 - c.h0);
         if (nh > nnarrow) {
@@ -1554,10 +1578,12 @@ void plan_execute(gsparc_plan *P, uint64_t chunk, uint64_t *keys, float *vals, u
     b.out_keys = keys;
     b.out_vals = vals;
     b.out_cap = c.n;
-    b.units = gp.units.get() + 2 * c.lu0;
-    b.nunits = (uint32_t)(c.lu1 - c.lu0);
+    b.units = gp.L.get();
+    b.nunits = (uint32_t)gp.nu;
+    b.l0 = (uint32_t)c.lu0;
+    b.l1 = (uint32_t)c.lu1;
     GS_CUDA(cudaMemsetAsync(gp.flags.get() + 1, 0, 4, s));
-    launch_light(b, true, (int)std::min<uint64_t>(gp.gl, std::max<uint64_t>(1, b.nunits)), s);
+    launch_light(b, kLightFinal, (int)std::min<uint64_t>(gp.gl, std::max<uint64_t>(1, b.nunits)), s);
     b.units = gp.heavy_list() + c.h0;
     b.nunits = (uint32_t)(c.h1 - c.h0);
     if (gp.nh > gp.nnarrow) {

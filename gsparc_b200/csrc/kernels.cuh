@@ -97,9 +97,17 @@ struct AccArgs {
     const uint32_t *row_xi;     // (of a narrow row: its number among the narrow rows)
     const uint64_t *sprefix;
     // work
-    const uint32_t *units;     // light: pairs (r0, r1); heavy and stream: row ids
-    uint32_t nunits;
+    const uint32_t *units;     // row ids
+    uint32_t nunits;           // rows (light: merge units in all)
     uint32_t light_cap;        // light: products of a unit stay below this (at most kLightCap)
+    uint64_t light_cols;       // light: column ranks are below this
+    // light rows [l0, l1) of the list (units holds it), their merge units and runs (rows.h)
+    uint32_t l0, l1;
+    const uint32_t *ustart, *lk0, *lrun, *lrow;
+    const uint64_t *lpre, *loff;
+    uint64_t *lpos;            // [light] first output of every light row in the scratch
+    uint64_t *lout_keys;       // scratch (kLightValues)
+    float *lout_vals;
     unsigned int *work_counter;
     uint32_t *cursor;          // [nx] scratch (heavy path): next unprocessed Y entry per run
     uint32_t *pend;            // [nx] scratch (heavy path): end of the run's part in the window
@@ -173,7 +181,9 @@ void launch_narrow(const AccArgs &a, bool numeric, int sm_count, cudaStream_t s)
 // numeric pass of single-run rows (their symbolic count is their product count)
 void launch_stream(const AccArgs &a, int grid, cudaStream_t s);
 int stream_blocks_per_sm();
-void launch_light(const AccArgs &a, bool numeric, int grid, cudaStream_t s);
+enum { kLightCount = 0, kLightValues = 1, kLightFinal = 2 };
+void launch_light(const AccArgs &a, int mode, int grid, cudaStream_t s);
+void launch_light_copy(const AccArgs &a, int sm_count, cudaStream_t s);
 int heavy_blocks_per_sm(bool numeric);
 int light_blocks_per_sm();
 

@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kScanThreads)
 __global__ void __launch_bounds__(kScanThreads)
     k_row_classes(const BPrep *__restrict__ jobs, const BatchJob *__restrict__ acc,
                   const uint64_t *__restrict__ range, RowArrays r, uint64_t *__restrict__ cnts, ScanState st) {
-    __shared__ ScanShared<4> sh;
+    __shared__ ScanShared<5> sh;
     if (ld_acquire(st.err) & kScanErr) return;
     const uint64_t nr = cnts[kCntRows];
     const uint32_t tile = next_tile(st, sh);
@@ -254,15 +254,19 @@ __global__ void __launch_bounds__(kScanThreads)
     const uint64_t i0 = (uint64_t)tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
     uint8_t cl[kScanItems];
     uint64_t pr[kScanItems];
-    uint64_t x[4] = {0, 0, 0, 0};  // heavy and (above 32 bits) stream rows; light and narrow rows; light, stream products
+    uint32_t rn[kScanItems];
+    // heavy and (above 32 bits) stream rows; light and narrow rows; light, stream products; light runs
+    uint64_t x[5] = {0, 0, 0, 0, 0};
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) {
         const uint64_t i = i0 + q;
         cl[q] = kRowNone;
         pr[q] = 0;
+        rn[q] = 0;
         if (i < nr) {
             pr[q] = r.xprefix[r.row_start[i + 1]] - r.xprefix[r.row_start[i]];
             const uint32_t k0 = r.row_k0[i], runs = r.row_k0[i + 1] - k0;
+            rn[q] = runs;
             if (i >= r0 && i < r1 && runs) {
                 const uint16_t j = r.row_job[i];
                 if (runs == 1 && !acc[j].ydup) {
@@ -285,9 +289,10 @@ __global__ void __launch_bounds__(kScanThreads)
             x[1] += (cl[q] == kRowLight) + ((uint64_t)(cl[q] == kRowNarrow) << 32);
             x[2] += cl[q] == kRowLight ? pr[q] : 0;
             x[3] += cl[q] == kRowStream ? pr[q] : 0;
+            x[4] += cl[q] == kRowLight ? rn[q] : 0;
         }
     }
-    if (!tile_scan<4>(st, sh, tile, x)) return;
+    if (!tile_scan<5>(st, sh, tile, x)) return;
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) {
         const uint32_t row = (uint32_t)(i0 + q);
@@ -304,11 +309,14 @@ __global__ void __launch_bounds__(kScanThreads)
             x[0] += 1ull << 32;
             x[3] += pr[q];
         } else if (cl[q] == kRowLight) {
-            r.L[(uint32_t)x[1]] = row;
-            r.lpre[(uint32_t)x[1]] = x[2];
-            r.lbrk[(uint32_t)x[1]] = (uint32_t)x[0] + (uint32_t)(x[0] >> 32);
+            const uint32_t l = (uint32_t)x[1];
+            r.L[l] = row;
+            r.row_xi[row] = l;
+            r.lpre[l] = x[2];
+            r.lk0[l] = (uint32_t)x[4];
             x[1] += 1;
             x[2] += pr[q];
+            x[4] += rn[q];
         }
     }
     if ((uint64_t)(tile + 1) * kScanTile >= nr && threadIdx.x == 0) {
@@ -316,13 +324,18 @@ __global__ void __launch_bounds__(kScanThreads)
         cnts[kCntStream] = sh.through[0] >> 32;
         cnts[kCntLight] = (uint32_t)sh.through[1];
         cnts[kCntNarrow] = sh.through[1] >> 32;
+        cnts[kCntLightProd] = sh.through[2];
+        r.lpre[(uint32_t)sh.through[1]] = sh.through[2];
+        r.lk0[(uint32_t)sh.through[1]] = (uint32_t)sh.through[4];
         r.sprefix[sh.through[0] >> 32] = sh.through[3];
     }
 }
 
-// A light unit is a maximal run of light rows whose first products fall in the
-// same bin of `bin` products, with no heavy or stream row between them (so it
-// is a contiguous row range): its products stay below bin + light_max.
+// A light unit is the light rows whose first products fall in the same bin of
+// `bin` products (counted over the light rows): its products stay below
+// bin + light_max.  Its rows need not be neighbours: rows of other classes
+// between them used to end a unit, which left units of one or two rows (157 to
+// 556 products) where single-run rows lie between the light ones.
 __global__ void __launch_bounds__(kScanThreads)
     k_light_units(uint64_t bin, RowArrays r, uint64_t *__restrict__ cnts, ScanState st) {
     __shared__ ScanShared<1> sh;
@@ -331,50 +344,37 @@ __global__ void __launch_bounds__(kScanThreads)
     const uint32_t tile = next_tile(st, sh);
     if ((uint64_t)tile * kScanTile >= n) return;
     const uint64_t i0 = (uint64_t)tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-    uint32_t starts = 0;  // bit q: a unit starts at light row i0 + q (bit kScanItems: at the one after)
-    uint64_t pb = 0;
-    uint32_t pk = 0;
-    if (i0 > 0 && i0 <= n) {
-        pb = r.lpre[i0 - 1] / bin;
-        pk = r.lbrk[i0 - 1];
-    }
-#pragma unroll
-    for (int q = 0; q <= kScanItems; ++q) {
-        const uint64_t i = i0 + q;
-        if (i < n) {
-            const uint64_t b = r.lpre[i] / bin;
-            const uint32_t k = r.lbrk[i];
-            if (i == 0 || b != pb || k != pk) starts |= 1u << q;
-            pb = b;
-            pk = k;
-        } else {
-            starts |= 1u << q;
-        }
-    }
-    uint64_t x[1] = {0};
-#pragma unroll
-    for (int q = 0; q < kScanItems; ++q) x[0] += i0 + q < n && (starts >> q & 1u);
-    if (!tile_scan<1>(st, sh, tile, x)) return;
+    uint32_t starts = 0;  // bit q: a unit starts at light row i0 + q
+    uint64_t pb = i0 > 0 && i0 < n ? r.lpre[i0 - 1] / bin : 0;
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) {
         const uint64_t i = i0 + q;
         if (i < n) {
-            const uint32_t row = r.L[i];
-            if (starts >> q & 1u) r.units[2 * x[0]++] = row;
-            if (starts >> (q + 1) & 1u) r.units[2 * (x[0] - 1) + 1] = row + 1;
+            const uint64_t b = r.lpre[i] / bin;
+            if (i == 0 || b != pb) starts |= 1u << q;
+            pb = b;
         }
     }
-    if ((uint64_t)(tile + 1) * kScanTile >= n && threadIdx.x == 0) cnts[kCntUnits] = sh.through[0];
+    uint64_t x[1] = {(uint64_t)__popc(starts)};
+    if (!tile_scan<1>(st, sh, tile, x)) return;
+#pragma unroll
+    for (int q = 0; q < kScanItems; ++q)
+        if (starts >> q & 1u) r.ustart[x[0]++] = (uint32_t)(i0 + q);
+    if ((uint64_t)(tile + 1) * kScanTile >= n && threadIdx.x == 0) {
+        cnts[kCntUnits] = sh.through[0];
+        r.ustart[sh.through[0]] = (uint32_t)n;
+    }
 }
 
-// Rank span of every heavy row: runs are sorted by rank, so a run's first and
-// last entries bound it.  A thread per matched X nonzero; a warp whose
-// nonzeros are of one row (long rows) folds them first.  With a warp per row,
-// 200 rows of 5e4 runs took 1155 us (200 warps at work); now 146.
-__global__ void k_heavy_spans(const uint32_t *__restrict__ pos, const uint32_t *__restrict__ cnt,
-                              const uint32_t *__restrict__ yrank, RowArrays r, const uint64_t *__restrict__ cnts,
-                              uint32_t *__restrict__ row_rb, uint32_t *__restrict__ row_mx,
-                              const unsigned int *__restrict__ err) {
+// A thread per matched X nonzero.  Light rows: their runs one after another,
+// with the products before each.  Heavy rows: the rank span (runs are sorted by
+// rank, so a run's first and last entries bound it); a warp whose nonzeros are
+// of one row (long rows) folds them first.  With a warp per row, 200 rows of
+// 5e4 runs took 1155 us (200 warps at work); now 146.
+__global__ void k_matched_runs(const uint32_t *__restrict__ pos, const uint32_t *__restrict__ cnt,
+                               const uint32_t *__restrict__ yrank, RowArrays r, const uint64_t *__restrict__ cnts,
+                               uint32_t *__restrict__ row_rb, uint32_t *__restrict__ row_mx,
+                               const unsigned int *__restrict__ err) {
     if (*err & kScanErr) return;
     const uint64_t n = r.row_k0[cnts[kCntRows]];  // matched nonzeros
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -382,7 +382,16 @@ __global__ void k_heavy_spans(const uint32_t *__restrict__ pos, const uint32_t *
     for (uint64_t k0 = t0 - (threadIdx.x & 31); k0 < n; k0 += stride) {  // whole warps
         const uint64_t k = k0 + (threadIdx.x & 31);
         const uint32_t row = r.mrow[k < n ? k : n - 1];
-        const bool heavy = k < n && r.row_class[row] == kRowHeavy;
+        const uint8_t cl = k < n ? r.row_class[row] : kRowNone;
+        if (cl == kRowLight) {
+            const uint32_t i = r.mrun[k], l = r.row_xi[row];
+            const uint32_t at = r.lk0[l] + (uint32_t)k - r.row_k0[row];
+            r.lrun[at] = i;
+            r.lrow[at] = l;
+            r.loff[at] = r.lpre[l] + r.xprefix[i] - r.xprefix[r.row_start[row]];
+        }
+        if (!row_rb) continue;  // the same in every thread
+        const bool heavy = cl == kRowHeavy;
         uint32_t lo = 0xffffffffu, hi = 0;
         if (heavy) {
             const uint32_t i = r.mrun[k], p = pos[i];
@@ -500,12 +509,18 @@ void launch_light_units(uint64_t nx, uint64_t bin, const RowArrays &r, uint64_t 
     launched();
 }
 
-void launch_heavy_bitmaps(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, const uint32_t *yrank,
-                          const RowArrays &r, uint32_t *row_rb, uint32_t *row_mx, uint32_t *w_all, uint32_t *w_dense,
-                          uint64_t *off_all, uint64_t *off_dense, uint64_t *cnts, const ScanState &st, cudaStream_t s) {
+void launch_matched_runs(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, const uint32_t *yrank,
+                         const RowArrays &r, uint32_t *row_rb, uint32_t *row_mx, const uint64_t *cnts,
+                         const unsigned int *err, cudaStream_t s) {
     if (nx == 0) return;
-    k_heavy_spans<<<grid_for(nx), kThreads, 0, s>>>(pos, cnt, yrank, r, cnts, row_rb, row_mx, st.err);
+    k_matched_runs<<<grid_for(nx), kThreads, 0, s>>>(pos, cnt, yrank, r, cnts, row_rb, row_mx, err);
     launched();
+}
+
+void launch_heavy_bitmaps(uint64_t nx, const RowArrays &r, const uint32_t *row_rb, const uint32_t *row_mx,
+                          uint32_t *w_all, uint32_t *w_dense, uint64_t *off_all, uint64_t *off_dense, uint64_t *cnts,
+                          const ScanState &st, cudaStream_t s) {
+    if (nx == 0) return;
     k_heavy_words<<<(unsigned)scan_tiles(nx), kScanThreads, 0, s>>>(r, row_rb, row_mx, w_all, w_dense, off_all,
                                                                     off_dense, cnts, st);
     launched();

@@ -26,6 +26,7 @@ enum {
     kCntUnits = 5,    // light units
     kCntMaxUnit = 6,  // largest unit output
     kCntStream = 7,
+    kCntLightProd = 8,  // products of the light rows
     kCntRange = 9,    // 9..11 shard row range and products
     kCntBmAll = 12,   // words of every kept bitmap
     kCntBmDense = 13, // words of the dense rows' kept bitmaps
@@ -65,12 +66,15 @@ struct RowArrays {
     uint64_t *row_prod;  // [nrows]
     uint8_t *row_class;  // [nrows]
     uint32_t *row_nnz;   // [nrows] stream rows: their products; 0 otherwise
-    uint32_t *row_xi;    // [nrows] stream rows: their matched X nonzero; narrow rows: their number
+    uint32_t *row_xi;    // [nrows] stream rows: their matched X nonzero; narrow and light rows: their number
     uint32_t *H, *SR, *L;  // heavy, stream and light rows, in row order
     uint64_t *sprefix;   // [stream + 1] products before every stream row
-    uint64_t *lpre;      // [light] products of the light rows before each one
-    uint32_t *lbrk;      // [light] heavy and stream rows before each light row
-    uint32_t *units;     // light units: row pairs
+    uint64_t *lpre;      // [light + 1] products of the light rows before each one
+    uint32_t *lk0;       // [light + 1] runs (matched X nonzeros) of the light rows before each one
+    uint32_t *ustart;    // [light units + 1] first light row (index into L) of every unit
+    uint32_t *lrun;      // [light runs] their X nonzeros, light row after light row
+    uint32_t *lrow;      // [light runs] their light rows (indices into L)
+    uint64_t *loff;      // [light runs] products of the light rows' runs before each one
 };
 // Match of every X nonzero -> prefix sums, matched list and rows.
 void launch_x_rows(const uint64_t *xkeys, uint64_t nx, int kbx, const BPrep *jobs, const uint32_t *cnt,
@@ -78,14 +82,18 @@ void launch_x_rows(const uint64_t *xkeys, uint64_t nx, int kbx, const BPrep *job
 // Row classes, their lists and product prefixes (rows outside `range` get no class).
 void launch_row_classes(uint64_t nx, const BPrep *jobs, const BatchJob *acc, const uint64_t *range,
                         const RowArrays &r, uint64_t *cnts, const ScanState &st, cudaStream_t s);
-// Light units of at most bin + light_max products.
+// Light units: consecutive light rows of fewer than bin + light_max products.
 void launch_light_units(uint64_t nx, uint64_t bin, const RowArrays &r, uint64_t *cnts, const ScanState &st,
                         cudaStream_t s);
-// Kept bitmaps: rank span of every heavy row, its words with all / only dense
+// The light rows' runs (lrun, lrow, loff) and, with row_rb (all ones at entry)
+// and row_mx (zeros), the rank span of every heavy row.
+void launch_matched_runs(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, const uint32_t *yrank,
+                         const RowArrays &r, uint32_t *row_rb, uint32_t *row_mx, const uint64_t *cnts,
+                         const unsigned int *err, cudaStream_t s);
+// Kept bitmaps: of every heavy row the words with all / only dense
 // rows kept (w_*, by row), their word offsets (off_*, by row) and totals.
-// row_rb must hold all ones and row_mx zeros for every heavy row.
-void launch_heavy_bitmaps(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, const uint32_t *yrank,
-                          const RowArrays &r, uint32_t *row_rb, uint32_t *row_mx, uint32_t *w_all, uint32_t *w_dense,
+void launch_heavy_bitmaps(uint64_t nx, const RowArrays &r, const uint32_t *row_rb, const uint32_t *row_mx,
+                          uint32_t *w_all, uint32_t *w_dense,
                           uint64_t *off_all, uint64_t *off_dense, uint64_t *cnts, const ScanState &st, cudaStream_t s);
 
 // unit_off[0..n] and part_off[0..n) of a heavy list (narrow.cu), units of about

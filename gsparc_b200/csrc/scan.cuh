@@ -29,6 +29,7 @@ inline uint64_t scan_tiles(uint64_t n) { return (n + kScanTile - 1) / kScanTile;
 
 // Words of a scan of at most n items: flags (zero at launch) and values.
 inline uint64_t scan_flag_words(uint64_t n) { return 1 + scan_tiles(n); }
+constexpr int kMaxScanSums = 5;  // sums of one scan (V) at most
 template <int V>
 uint64_t scan_value_words(uint64_t n) {
     return 2 * V * scan_tiles(n);
@@ -61,6 +62,7 @@ static __device__ __forceinline__ void st_release(uint32_t *p, uint32_t v) {
 template <int V>
 __device__ __forceinline__ bool look_back(const ScanState &st, uint32_t tile, const uint64_t (&tot)[V],
                                           uint64_t (&excl)[V]) {
+    static_assert(V <= kMaxScanSums, "the sums of a tile fit the buffer");
     const uint32_t lane = threadIdx.x & 31;
 #pragma unroll
     for (int v = 0; v < V; ++v) excl[v] = 0;

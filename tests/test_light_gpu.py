@@ -73,3 +73,63 @@ def test_light_rows(ctx, name, dup, light_max):
     assert np.array_equal(r.keys, z.keys)
     value_bar.max_rel_err(r.vals, z.vals)
     assert r.stats["heavy_rows"] == 0
+
+
+def _interleaved(rows):
+    """Light rows with single-run rows and a heavy row between them."""
+    out = []
+    for i, r in enumerate(rows):
+        out += [r, [7 + i % 5]]
+        if i % 37 == 11:
+            out.append([900, 800])
+    return out
+
+
+def test_interleaved_chunks_and_plan(ctx):
+    import torch
+    X, Y = _problem(_interleaved([[60, 40], [5, 5, 5], [300, 200, 9], [1, 2]] * 40), 11, 5000)
+    z = ob.sptc(X, Y, [1], [0])
+    for chunk in (0, 3000, 20011):
+        r = gb.SpTC(X, Y, [1], [0], ctx=ctx, max_chunk_nnz=chunk)
+        assert r.ir_nnz == z.ir_nnz and np.array_equal(r.keys, z.keys)
+        value_bar.max_rel_err(r.vals, z.vals)
+    dx, dy = ctx.upload(X), ctx.upload(Y)
+    p = gb.Plan(ctx, [(dx, dy, [1], [0])], max_chunk_nnz=3000)
+    keys, vals = torch.empty(z.nnz, dtype=torch.int64, device="cuda"), torch.empty(z.nnz, device="cuda")
+    p.refresh()
+    for k in range(p.nchunks):
+        f, n = p.chunk(k)
+        p.execute(k, keys[f:f + n], vals[f:f + n])
+    p.check()
+    assert p.nchunks > 5 and np.array_equal(keys.cpu().numpy().view(np.uint64), z.keys)
+    value_bar.max_rel_err(vals.cpu().numpy(), z.vals)
+    p.close()
+
+
+def test_without_scratch():
+    X, Y = _problem([[512, 500]] * 500, 3, 3000)
+    z = ob.sptc(X, Y, [1], [0])
+    with gb.Context(0, 24 << 20) as small:  # 6 MB of light products do not fit an eighth
+        r = gb.SpTC(X, Y, [1], [0], ctx=small)
+        assert r.ir_nnz == z.ir_nnz and np.array_equal(r.keys, z.keys)
+        value_bar.max_rel_err(r.vals, z.vals)
+
+
+@pytest.mark.parametrize("extra", [(1 << 20) - 4096, 1 << 20])
+def test_many_columns(ctx, extra):
+    """Ranks above and below 2^20: entries of 64 and of 32 bits."""
+    X, Y = _problem(CASES["odd_groups"], 5, 4096)
+    ncols = 4096 + extra
+    unused = Y.dims[0]
+    far = np.stack([np.full(extra, unused), 4096 + np.arange(extra)]).astype(np.uint64)
+    low = np.stack([np.full(4096, unused + 1), np.arange(4096)]).astype(np.uint64)
+    # the matched runs get the highest columns: mirror the free mode
+    idx = np.concatenate([Y.idx, far, low], axis=1)
+    idx[1] = ncols - 1 - idx[1]
+    val = np.concatenate([Y.val, np.ones(extra + 4096, np.float32)])
+    Y2 = gb.CooTensor([unused + 2, ncols], idx, val)
+    X2 = gb.CooTensor([X.dims[0], unused + 2], X.idx, X.val)
+    r = gb.SpTC(X2, Y2, [1], [0], ctx=ctx)
+    z = ob.sptc(X2, Y2, [1], [0])
+    assert r.ir_nnz == z.ir_nnz and np.array_equal(r.keys, z.keys)
+    value_bar.max_rel_err(r.vals, z.vals)
