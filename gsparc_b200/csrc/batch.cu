@@ -70,7 +70,8 @@ struct BLin {
     uint64_t nnz;
 };
 
-// Per-job summary after the symbolic pass (entry g holds the totals).
+// Per-job summary after the symbolic pass (entry g holds the totals, entry
+// g + 1 the largest output of one row and the error bits).
 struct JobOut {
     uint64_t row0;     // first row of the job
     uint64_t out_off;  // first output nonzero of the job
@@ -297,8 +298,9 @@ struct UnitLists {
 // Per-job summaries and the largest output of one unit.
 __global__ void k_after_counts(UnitLists u, const uint64_t *__restrict__ row_off, const uint16_t *__restrict__ row_job,
                                uint64_t nrows, const uint64_t *__restrict__ xprefix,
-                               const uint64_t *__restrict__ xoffs, int g, JobOut *__restrict__ jobs,
-                               uint64_t *__restrict__ out) {
+                               const uint64_t *__restrict__ xoffs, int g, const unsigned int *__restrict__ err,
+                               JobOut *__restrict__ jobs) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) jobs[g + 1].out_off = *err;
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j <= g; j += gridDim.x * blockDim.x) {
         const uint64_t r0 = (j == g) ? nrows : lower_bound_dev<uint16_t>(row_job, 0, nrows, (uint16_t)j);
         JobOut o;
@@ -320,7 +322,7 @@ __global__ void k_after_counts(UnitLists u, const uint64_t *__restrict__ row_off
         const uint64_t w = __shfl_xor_sync(0xffffffffu, m, o);
         m = w > m ? w : m;
     }
-    if ((threadIdx.x & 31) == 0 && m) atomicMax((unsigned long long *)out, (unsigned long long)m);
+    if ((threadIdx.x & 31) == 0 && m) atomicMax((unsigned long long *)&jobs[g + 1].row0, (unsigned long long)m);
 }
 
 // First row and first output of every unit, the three lists merged in row
@@ -426,8 +428,9 @@ struct GroupPlan {
     AccArgs aa{};
     std::vector<uint64_t> job_first;  // g + 1 group-local output offsets
     std::vector<Job *> jobs;
-    DBuf<BLin> d_lx, d_ly;
-    DBuf<uint64_t> d_xoffs, d_yoffs;
+    DBuf<uint8_t> tabs;
+    const BLin *d_lx = nullptr, *d_ly = nullptr;
+    const uint64_t *d_xoffs = nullptr, *d_yoffs = nullptr;
     DBuf<float> xperm, yperm, xvals, yvals;
     DBuf<uint64_t> ykeys;  // sorted Y keys (the single-run-row copy reads y_f from them)
     DBuf<BatchJob> d_acc;
@@ -533,90 +536,129 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     }
     const uint64_t nx = xoffs[g], ny = yoffs[g];
     // Column ranks through presence bits (and a prefix of their words) where
-    // these take at most 64 B per Y nonzero, or 4 MiB, and a sixteenth of the
+    // these take at most 64 B per Y nonzero, or 4 MiB, and a quarter of the
     // memory left; by sorting the free indices otherwise.  For 1.55e5 entries
     // over 2^24 free indices the scan and the lookups take 24 us (ncu) where the
     // sort, its unique and the searches took 60; for 1e7 entries over 300, 42
     // against 600.  The scan's time grows with the space (the bound keeps its
     // bytes within a few times those of the sort's passes over Y), and the
     // memory stays below the sort's two buffers except in the 4 MiB allowance.
-    const bool col_bits = col_words * 8 <= std::min(std::max<uint64_t>(64 * ny, 4ull << 20), A.available() / 16);
+    // What the planning needs in any case comes first.
+    const uint64_t plan_need = 192 * nx + 96 * ny + (8ull << 20);
+    const uint64_t table_most = std::min(std::max<uint64_t>(64 * ny, 4ull << 20),
+                                         (A.available() - std::min(A.available(), plan_need)) / 4);
+    const bool col_bits = col_words * 8 <= table_most;
     // The run lookup table (8 B per 32 contract keys) under the same bounds.
     // With it the match does not care for the order of a row's nonzeros, so X
     // is sorted by its free bits alone.  1e7 x 1e7 nonzeros over 2^24 contract
     // keys: X's radix passes 4 -> 1 (122 us each), match 241 -> 101 us.
-    const bool con_tab = con_words * 8 <= std::min(std::max<uint64_t>(64 * ny, 4ull << 20), A.available() / 16);
-    DBuf<BLin> d_lx(A, g, s), d_ly(A, g, s);
-    DBuf<BPrep> d_bp(A, g, s);
+    const bool con_tab = con_words * 8 <= table_most;
+    // the job tables, copied at once
+    const size_t o_ly = sizeof(BLin) * g, o_bp = 2 * o_ly, o_xo = o_bp + sizeof(BPrep) * g,
+                 o_yo = o_xo + 8 * (size_t)(g + 1), tab_bytes = o_yo + 8 * (size_t)(g + 1);
+    static_assert(sizeof(BLin) % 8 == 0 && sizeof(BPrep) % 8 == 0, "8-byte aligned tables");
+    DBuf<uint8_t> tabs(A, tab_bytes, s);
+    const BLin *const d_lx = reinterpret_cast<const BLin *>(tabs.get()),
+               *const d_ly = reinterpret_cast<const BLin *>(tabs.get() + o_ly);
+    const BPrep *const d_bp = reinterpret_cast<const BPrep *>(tabs.get() + o_bp);
+    const uint64_t *const d_xoffs = reinterpret_cast<const uint64_t *>(tabs.get() + o_xo),
+                   *const d_yoffs = reinterpret_cast<const uint64_t *>(tabs.get() + o_yo);
     DBuf<BatchJob> d_acc(A, g, s);
-    DBuf<uint64_t> d_xoffs(A, g + 1, s), d_yoffs(A, g + 1, s);
     // what starts at zero, cleared at once: the counters (kCnt*), the run lookup
     // table, the jobs' error and repeated-coordinate words, the scans' flags, the presence bits
     const uint64_t zf_y = scan_flag_words(ny), zf_c = col_bits ? scan_flag_words(col_words) : 0,
                    zf_x = scan_flag_words(nx);
     const uint64_t tab_words = con_tab ? 2 * con_words : 0;
-    const uint64_t zwords = 2 * kCnts + tab_words + 2 * (uint64_t)g + zf_y + zf_c + 6 * zf_x + (col_bits ? col_words : 0);
+    // counters, jobs' error and repeated-coordinate words (an even number of
+    // words), run table, job summaries, flags, bits
+    const uint64_t zw_jobs = 2 * (uint64_t)g, zw_out = sizeof(JobOut) / 4 * (uint64_t)(g + 2);
+    const uint64_t zwords = 2 * kCnts + zw_jobs + tab_words + zw_out + zf_y + zf_c + 6 * zf_x + (col_bits ? col_words : 0);
     DBuf<uint32_t> zero(A, zwords, s);
     uint64_t *const cnts = reinterpret_cast<uint64_t *>(zero.get());
-    uint2 *const ctab = con_tab ? reinterpret_cast<uint2 *>(zero.get() + 2 * kCnts) : nullptr;
-    unsigned int *const d_jerr = zero.get() + 2 * kCnts + tab_words, *const d_ydup = d_jerr + g;
-    uint32_t *const flags_y = d_ydup + g, *const flags_c = flags_y + zf_y, *const flags_x = flags_c + zf_c;
+    unsigned int *const d_jerr = zero.get() + 2 * kCnts, *const d_ydup = d_jerr + g;
+    unsigned int *const plan_err = reinterpret_cast<unsigned int *>(cnts + kCntErr);
+    uint2 *const ctab = con_tab ? reinterpret_cast<uint2 *>(zero.get() + 2 * kCnts + zw_jobs) : nullptr;
+    JobOut *const d_jo = reinterpret_cast<JobOut *>(zero.get() + 2 * kCnts + zw_jobs + tab_words);
+    uint32_t *const flags_y = zero.get() + 2 * kCnts + zw_jobs + tab_words + zw_out, *const flags_c = flags_y + zf_y,
+                    *const flags_x = flags_c + zf_c;
     uint32_t *const ybits = col_bits ? flags_x + 6 * zf_x : nullptr;
     // the scans' sums (one buffer: the scans follow one another on the stream)
     DBuf<uint64_t> scan_vals(A, std::max({scan_value_words<1>(ny), col_bits ? scan_value_words<1>(col_words) : 0,
                                           scan_value_words<kMaxScanSums>(nx)}), s);
-    auto scan_state = [&](uint32_t *flags) { return ScanState{flags, scan_vals.get(), ctx->d_flag}; };
-    h2d(d_lx.get(), lx.data(), g, s);
-    h2d(d_ly.get(), ly.data(), g, s);
-    h2d(d_bp.get(), bp.data(), g, s);
-    h2d(d_xoffs.get(), xoffs.data(), g + 1, s);
-    h2d(d_yoffs.get(), yoffs.data(), g + 1, s);
+    auto scan_state = [&](uint32_t *flags) { return ScanState{flags, scan_vals.get(), plan_err}; };
+    std::vector<uint8_t> h_tabs(tab_bytes);
+    std::memcpy(h_tabs.data(), lx.data(), o_ly);
+    std::memcpy(h_tabs.data() + o_ly, ly.data(), o_ly);
+    std::memcpy(h_tabs.data() + o_bp, bp.data(), sizeof(BPrep) * g);
+    std::memcpy(h_tabs.data() + o_xo, xoffs.data(), 8 * (size_t)(g + 1));
+    std::memcpy(h_tabs.data() + o_yo, yoffs.data(), 8 * (size_t)(g + 1));
+    h2d(tabs.get(), h_tabs.data(), tab_bytes, s);
     GS_CUDA(cudaMemsetAsync(zero.get(), 0, 4 * zwords, s));
     GS_CUDA(cudaMemsetAsync(ctx->d_flag, 0, 4 * 4, s));
     bst.bytes_h2d += (sizeof(BLin) * 2 + sizeof(BPrep) + 16) * g;
 
-    // ---- linearise ----
+    // ---- linearise and sort ----
+    // X's on the other stream: it is needed at the match, while Y's tables are
+    // made on this one.  Its buffers are this stream's, so they are given back
+    // only after the join; an error before it waits for the other stream.
     DBuf<uint64_t> xk0(A, nx, s), xk1(A, nx, s), yk0(A, ny, s), yk1(A, ny, s);
     DBuf<float> xv0(A, nx, s), xv1(A, nx, s), yv0(A, ny, s), yv1(A, ny, s);
+    if (keep) {
+        keep->xvals.reset(A, std::max<uint64_t>(nx, 1), s);
+        keep->yvals.reset(A, std::max<uint64_t>(ny, 1), s);
+    }
+    const cudaStream_t sx = ctx->alt_stream ? ctx->alt_stream : s;
+    struct Join {
+        cudaStream_t sx = nullptr;
+        ~Join() {
+            if (sx) cudaStreamSynchronize(sx);
+        }
+    } join;
+    GS_CUDA(cudaEventRecord(ev[8], s));
+    GS_CUDA(cudaStreamWaitEvent(sx, ev[8], 0));
+    join.sx = sx;
+    const int xbegin = con_tab ? min_ncb : 0;
+    int wx = 0, wy = 0;
     if (nx) {
-        k_blin<<<grid_for(nx), kThreads, 0, s>>>(d_lx, d_xoffs, g, nx, kbx, xk0, xv0, d_jerr, keep != nullptr);
+        k_blin<<<grid_for(nx), kThreads, 0, sx>>>(d_lx, d_xoffs, g, nx, kbx, xk0, xv0, d_jerr, keep != nullptr);
         count_launch();
         GS_CUDA(cudaGetLastError());
     }
+    // gsparc_ctx_set_sort; a failed look-back sets bit 8 of the error word
+    if (ctx->sort_impl)
+        own_sort_pairs(A, nx, xk0, xk1, xv0, xv1, kbx + jb, &wx, plan_err, sx, xbegin);
+    else
+        sort_pairs(A, nx, xk0, xk1, xv0, xv1, kbx + jb, &wx, sx, xbegin);
+    if (keep && nx) {
+        k_bvals<<<grid_for(nx), kThreads, 0, sx>>>(d_lx, d_xoffs, g, nx, wx ? xv1 : xv0, keep->xvals);
+        count_launch();
+        GS_CUDA(cudaGetLastError());
+    }
+    GS_CUDA(cudaEventRecord(ev[9], sx));
     if (ny) {
         k_blin<<<grid_for(ny), kThreads, 0, s>>>(d_ly, d_yoffs, g, ny, kby, yk0, yv0, d_jerr, keep != nullptr);
         count_launch();
         GS_CUDA(cudaGetLastError());
     }
     mark(1);
-
-    // ---- sort ----
-    int wx = 0, wy = 0;
-    const int xbegin = con_tab ? min_ncb : 0;
-    if (ctx->sort_impl) {  // gsparc_ctx_set_sort; a failed look-back sets bit 8 of the error word
-        own_sort_pairs(A, nx, xk0, xk1, xv0, xv1, kbx + jb, &wx, ctx->d_flag, s, xbegin);
-        own_sort_pairs(A, ny, yk0, yk1, yv0, yv1, kby + jb, &wy, ctx->d_flag, s);
-    } else {
-        sort_pairs(A, nx, xk0, xk1, xv0, xv1, kbx + jb, &wx, s, xbegin);
+    if (ctx->sort_impl)
+        own_sort_pairs(A, ny, yk0, yk1, yv0, yv1, kby + jb, &wy, plan_err, s);
+    else
         sort_pairs(A, ny, yk0, yk1, yv0, yv1, kby + jb, &wy, s);
-    }
     const uint64_t *xkeys = wx ? xk1.get() : xk0.get();
     const float *xvals = wx ? xv1.get() : xv0.get();
     const uint64_t *ykeys = wy ? yk1.get() : yk0.get();
     const float *yvals = wy ? yv1.get() : yv0.get();
-    if (wx) { xk0.release(); xv0.release(); } else { xk1.release(); xv1.release(); }
     if (wy) { yk0.release(); yv0.release(); } else { yk1.release(); yv1.release(); }
     if (keep) {
         // the sorted "values" are input positions: keep them, fetch the values
         keep->ykeys = wy ? std::move(yk1) : std::move(yk0);  // ykeys keeps pointing at it
-        keep->xperm = wx ? std::move(xv1) : std::move(xv0);
         keep->yperm = wy ? std::move(yv1) : std::move(yv0);
-        keep->xvals.reset(A, std::max<uint64_t>(nx, 1), s);
-        keep->yvals.reset(A, std::max<uint64_t>(ny, 1), s);
-        if (nx) k_bvals<<<grid_for(nx), kThreads, 0, s>>>(d_lx, d_xoffs, g, nx, keep->xperm, keep->xvals);
-        if (ny) k_bvals<<<grid_for(ny), kThreads, 0, s>>>(d_ly, d_yoffs, g, ny, keep->yperm, keep->yvals);
-        count_launch((nx ? 1 : 0) + (ny ? 1 : 0));
-        GS_CUDA(cudaGetLastError());
+        if (ny) {
+            k_bvals<<<grid_for(ny), kThreads, 0, s>>>(d_ly, d_yoffs, g, ny, keep->yperm, keep->yvals);
+            count_launch();
+            GS_CUDA(cudaGetLastError());
+        }
         xvals = keep->xvals.get();
         yvals = keep->yvals.get();
     }
@@ -631,7 +673,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         launch_y_runs(ykeys, ny, kby, d_bp, run_key, run_start, cnts, d_ydup, ybits, nullptr, ctab, scan_state(flags_y), s);
         DBuf<uint32_t> wpre(A, col_words, s);
         launch_col_table(ybits, col_words, d_bp, g, wpre, cols, cnts, scan_state(flags_c), s);
-        launch_y_ranks(ykeys, ny, kby, d_bp, g, ybits, wpre, cnts, rank, d_acc, d_ydup, ctx->d_flag, s);
+        launch_y_ranks(ykeys, ny, kby, d_bp, g, ybits, wpre, cnts, rank, d_acc, d_ydup, plan_err, s);
     } else {
         DBuf<uint64_t> yf0(A, nyb, s), yf1(A, nyb, s);
         launch_y_runs(ykeys, ny, kby, d_bp, run_key, run_start, cnts, d_ydup, nullptr, yf0, ctab, scan_state(flags_y), s);
@@ -658,6 +700,10 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     }
 
     // ---- X match, row table and unit planning ----
+    GS_CUDA(cudaStreamWaitEvent(s, ev[9], 0));
+    join.sx = nullptr;
+    if (wx) { xk0.release(); xv0.release(); } else { xk1.release(); xv1.release(); }
+    if (keep) keep->xperm = wx ? std::move(xv1) : std::move(xv0);
     DBuf<uint32_t> pos(A, nxb, s), cnt(A, nxb, s);
     DBuf<uint64_t> xprefix(A, nx + 1, s);
     DBuf<uint32_t> row_start(A, nx + 1, s);
@@ -716,7 +762,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         const uint64_t *range = nullptr;
         if (nshards > 1) {
             k_shard_range<<<1, 32, 0, s>>>(xprefix, row_start, cnts + kCntRows, shard, nshards, cnts + kCntRange,
-                                           ctx->d_flag);
+                                           plan_err);
             count_launch();
             GS_CUDA(cudaGetLastError());
             range = cnts + kCntRange;
@@ -730,7 +776,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
             GS_CUDA(cudaMemsetAsync(row_rb.get(), 0xff, 4 * nx, s));
             GS_CUDA(cudaMemsetAsync(row_mx.get(), 0, 4 * nx, s));
         }
-        launch_matched_runs(nx, pos, cnt, rank, ra, row_rb, row_mx, cnts, ctx->d_flag, s);
+        launch_matched_runs(nx, pos, cnt, rank, ra, row_rb, row_mx, cnts, plan_err, s);
         if (keep_bm)
             launch_heavy_bitmaps(nx, ra, row_rb, row_mx, bm_w_all, bm_w_dense, bm_off_all, bm_off_dense, cnts,
                                  scan_state(flags_x + 3 * zf_x), s);
@@ -740,15 +786,22 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         GS_CUDA(cudaMemsetAsync(row_start.get(), 0, 4, s));
         mark(3);
     }
-    uint64_t hc_cnt[kCnts];
-    std::vector<unsigned int> jerr(g);
-    uint64_t ir = 0;
-    unsigned int herr = 0;
-    d2h(hc_cnt, cnts, kCnts, s);
-    d2h(jerr.data(), d_jerr, g, s);
-    d2h(&ir, xprefix.get() + nx, 1, s);
-    d2h(&herr, ctx->d_flag, 1, s);
+    // counters and the jobs' error words, copied at once
+    const size_t head_bytes = 8 * kCnts + 4 * (size_t)g;
+    std::vector<uint8_t> h_head;
+    uint8_t *head = static_cast<uint8_t *>(ctx->h_pin);
+    if (!head || head_bytes > gsparc_ctx::kPinBytes) {
+        h_head.resize(head_bytes);
+        head = h_head.data();
+    }
+    d2h(head, reinterpret_cast<const uint8_t *>(zero.get()), head_bytes, s);
     GS_CUDA(cudaStreamSynchronize(s));
+    uint64_t hc_cnt[kCnts];
+    std::memcpy(hc_cnt, head, sizeof(hc_cnt));
+    std::vector<unsigned int> jerr(g);
+    std::memcpy(jerr.data(), head + sizeof(hc_cnt), 4 * (size_t)g);
+    unsigned int herr = (unsigned int)hc_cnt[kCntErr];
+    uint64_t ir = hc_cnt[kCntProducts];
     GS_REQUIRE(!(herr & kScanErr), GSPARC_EINTERNAL, "a prefix sum's or the radix sort's look-back gave up");
     const uint64_t bm_words_all = hc_cnt[kCntBmAll], bm_words_dense = hc_cnt[kCntBmDense];
     const uint64_t nrows = hc_cnt[kCntRows], nh = hc_cnt[kCntHeavy], nl = hc_cnt[kCntLight],
@@ -767,7 +820,13 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
                                               1ull << 20);
     const uint64_t narrow_cols = hc_cnt[kCntNarrowCols], nbm_words = hc_cnt[kCntNarrow] * (kNarrowCols / 32),
                    nparts = 2 * (ir / slice) * narrow_cols;
-    const uint64_t nnarrow = 4 * nbm_words + 8 * nparts <= A.available() / 16 ? hc_cnt[kCntNarrow] : 0;
+    // the output of the widest row, twice in two chunks, and the heavy rows'
+    // cursors must fit beside what is optional
+    const uint64_t out_need = 48 * hc_cnt[kCntCols] + 16 * nx + (1ull << 20);
+    const auto fits = [&](uint64_t bytes, uint64_t part) {
+        return bytes <= A.available() / part && bytes + out_need <= A.available();
+    };
+    const uint64_t nnarrow = fits(4 * nbm_words + 8 * nparts, 16) ? hc_cnt[kCntNarrow] : 0;
     const uint8_t *narrow_class = nnarrow ? row_class.get() : nullptr;
 
     // heavy rows largest first (H itself stays in row order for chunk planning)
@@ -814,7 +873,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     // time in place) where that does not fit an eighth of the memory left, and
     // for plans, whose values change.
     const uint64_t light_prod = hc_cnt[kCntLightProd];
-    const bool light_once = !keep && nu && light_prod * 12 <= A.available() / 8;
+    const bool light_once = !keep && nu && fits(12 * light_prod, 8);
     DBuf<uint64_t> lout_keys, lpos;
     DBuf<float> lout_vals;
     if (light_once) {
@@ -911,18 +970,19 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         }
     }
     exclusive_scan_u32_to_u64(A, row_nnz, row_off, nrows, s);
-    DBuf<JobOut> d_jo(A, g + 1, s);
     const UnitLists ul{L, nl, H, nh, SR, nsr};
     k_after_counts<<<grid_for(std::max<uint64_t>(nl + nh + nsr, (uint64_t)g + 1)), kThreads, 0, s>>>(
-        ul, row_off, row_job, nrows, xprefix, d_xoffs, g, d_jo, cnts + kCntMaxUnit);
+        ul, row_off, row_job, nrows, xprefix, d_xoffs, g, ctx->d_flag, d_jo);
     count_launch();
     GS_CUDA(cudaGetLastError());
-    std::vector<JobOut> jo(g + 1);
-    uint64_t max_unit = 0;
-    d2h(jo.data(), d_jo.get(), g + 1, s);
-    d2h(&herr, ctx->d_flag, 1, s);
-    d2h(&max_unit, cnts + kCntMaxUnit, 1, s);
+    std::vector<JobOut> jo(g + 2);
+    const size_t jo_bytes = sizeof(JobOut) * (size_t)(g + 2);
+    void *jo_at = ctx->h_pin && jo_bytes <= gsparc_ctx::kPinBytes ? ctx->h_pin : jo.data();
+    d2h(static_cast<uint8_t *>(jo_at), reinterpret_cast<const uint8_t *>(d_jo), jo_bytes, s);
     GS_CUDA(cudaStreamSynchronize(s));
+    if (jo_at != jo.data()) std::memcpy(jo.data(), jo_at, jo_bytes);
+    const uint64_t max_unit = jo[g + 1].row0;
+    herr = (unsigned int)jo[g + 1].out_off;
     bst.bytes_d2h += sizeof(JobOut) * (g + 1) + 64 + 4 * g + 8;
     GS_REQUIRE(!(herr & 2u), GSPARC_EINTERNAL, "light unit over capacity");
     const uint64_t ntot = jo[g].out_off;
@@ -1049,10 +1109,11 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         keep->job_first.resize(g + 1);
         for (int j = 0; j <= g; ++j) keep->job_first[j] = jo[j].out_off;
         keep->jobs = G;
-        keep->d_lx = std::move(d_lx);
-        keep->d_ly = std::move(d_ly);
-        keep->d_xoffs = std::move(d_xoffs);
-        keep->d_yoffs = std::move(d_yoffs);
+        keep->d_lx = d_lx;  // in tabs
+        keep->d_ly = d_ly;
+        keep->d_xoffs = d_xoffs;
+        keep->d_yoffs = d_yoffs;
+        keep->tabs = std::move(tabs);
         keep->d_acc = std::move(d_acc);
         keep->rank = std::move(rank);
         keep->pos = std::move(pos);
@@ -1295,7 +1356,8 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         }
     }
     mark(5);
-    unsigned int hflags[4] = {0, 0, 0, 0};
+    unsigned int hflags_own[4] = {0, 0, 0, 0};
+    unsigned int *hflags = ctx->h_pin ? static_cast<unsigned int *>(ctx->h_pin) : hflags_own;
     d2h(hflags, ctx->d_flag, 4, s);
     GS_CUDA(cudaStreamSynchronize(s));
     bst.heavy_windows += hflags[2];

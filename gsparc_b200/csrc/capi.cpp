@@ -86,6 +86,7 @@ gsparc_status gsparc_ctx_create(int device, uint64_t budget, gsparc_ctx **out) {
             GS_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
             GS_CUDA(cudaStreamCreateWithFlags(&ctx->alt_stream, cudaStreamNonBlocking));
             GS_CUDA(cudaMemset(ctx->d_flag, 0, 64));
+            GS_CUDA(cudaMallocHost(&ctx->h_pin, gsparc_ctx::kPinBytes));
         } catch (...) {
             delete ctx;
             throw;
@@ -104,6 +105,7 @@ gsparc_status gsparc_ctx_destroy(gsparc_ctx *ctx) {
         if (ctx->d_flag) cudaFree(ctx->d_flag);
         if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
         if (ctx->alt_stream) cudaStreamDestroy(ctx->alt_stream);
+        if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
         delete ctx;
     });
 }

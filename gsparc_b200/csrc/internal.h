@@ -146,7 +146,9 @@ struct gsparc_ctx {
     cudaEvent_t ev[16] = {};
     unsigned int *d_flag = nullptr;  // device error / work counters
     cudaStream_t copy_stream = nullptr;  // output chunk copies (non-blocking)
-    cudaStream_t alt_stream = nullptr;   // every other output chunk's kernels (non-blocking)
+    cudaStream_t alt_stream = nullptr;   // every other output chunk's kernels, X's linearise and sort (non-blocking)
+    void *h_pin = nullptr;               // page-locked landing place of small readbacks
+    static constexpr size_t kPinBytes = 1 << 16;
     uint64_t verify_budget = 0;          // FP64 verification of outputs (0: off)
     uint64_t light_row_max = 0;          // rows with at most this many products use the on-chip ESC (0: default)
     uint32_t heavy_window_cap = 0;       // heavy rows: outputs per window (0: the compiled capacity)

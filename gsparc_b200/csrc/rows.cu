@@ -235,6 +235,7 @@ __global__ void __launch_bounds__(kScanThreads)
         r.row_start[nr] = (uint32_t)nx;
         r.row_k0[nr] = nm;
         cnts[kCntRows] = nr;
+        cnts[kCntProducts] = sh.through[0];
     }
 }
 

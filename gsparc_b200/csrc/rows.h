@@ -24,7 +24,6 @@ enum {
     kCntHeavy = 3,
     kCntLight = 4,    // light rows
     kCntUnits = 5,    // light units
-    kCntMaxUnit = 6,  // largest unit output
     kCntStream = 7,
     kCntLightProd = 8,  // products of the light rows
     kCntRange = 9,    // 9..11 shard row range and products
@@ -32,7 +31,9 @@ enum {
     kCntBmDense = 13, // words of the dense rows' kept bitmaps
     kCntNarrow = 14,     // narrow rows among the heavy ones
     kCntNarrowCols = 15, // most columns of a job with narrow rows
-    kCnts = 16
+    kCntProducts = 16,
+    kCntErr = 17,        // error bits of the planning kernels and the radix sort (low word)
+    kCnts = 18
 };
 
 constexpr uint8_t kRowNone = 0, kRowLight = 1, kRowStream = 2, kRowHeavy = 3, kRowNarrow = 4;  // narrow: heavy, over few columns
