@@ -158,6 +158,7 @@ __global__ void k_bjobs(const uint64_t *__restrict__ uniq, const uint64_t *__res
         b.y_nfbits = jobs[j].y_nfbits;
         b.ncols = (uint32_t)(hi - lo);
         b.ydup = ydup[j];
+        b.wide = 0;
         b.cols_off = lo;
         acc[j] = b;
     }
@@ -553,9 +554,13 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     // is sorted by its free bits alone.  1e7 x 1e7 nonzeros over 2^24 contract
     // keys: X's radix passes 4 -> 1 (122 us each), match 241 -> 101 us.
     const bool con_tab = con_words * 8 <= table_most;
+    // relabeled jobs with 64-bit output keys
+    bool any_wide = false;
+    for (Job *q : G) any_wide |= q->wide && q->key_words == 1;
     // the job tables, copied at once
     const size_t o_ly = sizeof(BLin) * g, o_bp = 2 * o_ly, o_xo = o_bp + sizeof(BPrep) * g,
-                 o_yo = o_xo + 8 * (size_t)(g + 1), tab_bytes = o_yo + 8 * (size_t)(g + 1);
+                 o_yo = o_xo + 8 * (size_t)(g + 1), o_wt = o_yo + 8 * (size_t)(g + 1),
+                 tab_bytes = o_wt + sizeof(WideTab) * (any_wide ? g : 0);
     static_assert(sizeof(BLin) % 8 == 0 && sizeof(BPrep) % 8 == 0, "8-byte aligned tables");
     DBuf<uint8_t> tabs(A, tab_bytes, s);
     const BLin *const d_lx = reinterpret_cast<const BLin *>(tabs.get()),
@@ -570,9 +575,10 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
                    zf_x = scan_flag_words(nx);
     const uint64_t tab_words = con_tab ? 2 * con_words : 0;
     // counters, jobs' error and repeated-coordinate words (an even number of
-    // words), run table, job summaries, flags, bits
+    // words), run table, job summaries, flags, the work counters of the symbolic pass and the first chunk, bits
+    constexpr uint64_t zw_work = 6;
     const uint64_t zw_jobs = 2 * (uint64_t)g, zw_out = sizeof(JobOut) / 4 * (uint64_t)(g + 2);
-    const uint64_t zwords = 2 * kCnts + zw_jobs + tab_words + zw_out + zf_y + zf_c + 6 * zf_x + (col_bits ? col_words : 0);
+    const uint64_t zwords = 2 * kCnts + zw_jobs + tab_words + zw_out + zf_y + zf_c + 7 * zf_x + zw_work + (col_bits ? col_words : 0);
     DBuf<uint32_t> zero(A, zwords, s);
     uint64_t *const cnts = reinterpret_cast<uint64_t *>(zero.get());
     unsigned int *const d_jerr = zero.get() + 2 * kCnts, *const d_ydup = d_jerr + g;
@@ -581,7 +587,8 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     JobOut *const d_jo = reinterpret_cast<JobOut *>(zero.get() + 2 * kCnts + zw_jobs + tab_words);
     uint32_t *const flags_y = zero.get() + 2 * kCnts + zw_jobs + tab_words + zw_out, *const flags_c = flags_y + zf_y,
                     *const flags_x = flags_c + zf_c;
-    uint32_t *const ybits = col_bits ? flags_x + 6 * zf_x : nullptr;
+    unsigned int *const work = flags_x + 7 * zf_x;
+    uint32_t *const ybits = col_bits ? work + zw_work : nullptr;
     // the scans' sums (one buffer: the scans follow one another on the stream)
     DBuf<uint64_t> scan_vals(A, std::max({scan_value_words<1>(ny), col_bits ? scan_value_words<1>(col_words) : 0,
                                           scan_value_words<kMaxScanSums>(nx)}), s);
@@ -592,6 +599,13 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     std::memcpy(h_tabs.data() + o_bp, bp.data(), sizeof(BPrep) * g);
     std::memcpy(h_tabs.data() + o_xo, xoffs.data(), 8 * (size_t)(g + 1));
     std::memcpy(h_tabs.data() + o_yo, yoffs.data(), 8 * (size_t)(g + 1));
+    if (any_wide)
+        for (int j = 0; j < g; ++j) {
+            WideTab t{};
+            if (G[j]->wide && G[j]->key_words == 1)
+                t = {G[j]->wide->xf.get(), G[j]->wide->yf.get(), G[j]->wide->nfbits_y, 0};
+            std::memcpy(h_tabs.data() + o_wt + sizeof(WideTab) * j, &t, sizeof(t));
+        }
     h2d(tabs.get(), h_tabs.data(), tab_bytes, s);
     GS_CUDA(cudaMemsetAsync(zero.get(), 0, 4 * zwords, s));
     GS_CUDA(cudaMemsetAsync(ctx->d_flag, 0, 4 * 4, s));
@@ -758,7 +772,16 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         ra.lrun = lrun;
         ra.lrow = lrow;
         ra.loff = loff;
+        DBuf<uint32_t> row_mx;
+        if (keep_bm) {
+            row_mx.reset(A, nx, s);
+            ra.row_rb = row_rb;
+            ra.row_mx = row_mx;
+        }
         launch_x_rows(xkeys, nx, kbx, d_bp, cnt, rflag, ra, cnts, scan_state(flags_x), s);
+        if (any_wide)
+            launch_wide_tables(reinterpret_cast<const WideTab *>(tabs.get() + o_wt), g, std::max(nx, ny), row_job, row_xf,
+                               cols, d_acc, cnts, plan_err, s);
         const uint64_t *range = nullptr;
         if (nshards > 1) {
             k_shard_range<<<1, 32, 0, s>>>(xprefix, row_start, cnts + kCntRows, shard, nshards, cnts + kCntRange,
@@ -770,15 +793,9 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         launch_row_classes(nx, d_bp, d_acc, range, ra, cnts, scan_state(flags_x + zf_x), s);
         mark(3);
         launch_light_units(nx, light_bin, ra, cnts, scan_state(flags_x + 2 * zf_x), s);
-        DBuf<uint32_t> row_mx;
-        if (keep_bm) {
-            row_mx.reset(A, nx, s);
-            GS_CUDA(cudaMemsetAsync(row_rb.get(), 0xff, 4 * nx, s));
-            GS_CUDA(cudaMemsetAsync(row_mx.get(), 0, 4 * nx, s));
-        }
-        launch_matched_runs(nx, pos, cnt, rank, ra, row_rb, row_mx, cnts, plan_err, s);
+        launch_matched_runs(nx, pos, cnt, rank, ra, cnts, plan_err, s);
         if (keep_bm)
-            launch_heavy_bitmaps(nx, ra, row_rb, row_mx, bm_w_all, bm_w_dense, bm_off_all, bm_off_dense, cnts,
+            launch_heavy_bitmaps(nx, ra, bm_w_all, bm_w_dense, bm_off_all, bm_off_dense, cnts,
                                  scan_state(flags_x + 3 * zf_x), s);
     } else {
         GS_CUDA(cudaMemsetAsync(xprefix.get(), 0, 8, s));
@@ -889,6 +906,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     aa.yval = yvals;
     aa.ykeys = ykeys;
     aa.cols = cols;
+    aa.any_wide = any_wide;
     aa.work_counter = ctx->d_flag + 1;
     aa.cursor = cursor;
     aa.pend = pend;
@@ -954,22 +972,22 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         b.nunits = (uint32_t)nu;
         b.l0 = 0;
         b.l1 = (uint32_t)nl;
-        GS_CUDA(cudaMemsetAsync(ctx->d_flag + 1, 0, 4, s));
+        b.work_counter = work;
         b.out_cap = light_prod;
         launch_light(b, light_once ? kLightValues : kLightCount,
                      (int)std::min<uint64_t>(gl, std::max<uint64_t>(1, nu)), s);
         b.units = Hs;
         b.nunits = (uint32_t)nh;
         if (nh > nnarrow) {
-            GS_CUDA(cudaMemsetAsync(ctx->d_flag + 1, 0, 4, s));
+            b.work_counter = work + 1;
             launch_heavy(b, false, (int)std::min<uint64_t>(ghs, std::max<uint64_t>(1, nh)), s);
         }
         if (nnarrow) {
-            GS_CUDA(cudaMemsetAsync(ctx->d_flag + 1, 0, 4, s));
+            b.work_counter = work + 2;
             launch_narrow(b, false, ctx->sm_count, s);
         }
     }
-    exclusive_scan_u32_to_u64(A, row_nnz, row_off, nrows, s);
+    launch_row_offsets(row_nnz, nrows, row_off, scan_state(flags_x + 6 * zf_x), s);
     const UnitLists ul{L, nl, H, nh, SR, nsr};
     k_after_counts<<<grid_for(std::max<uint64_t>(nl + nh + nsr, (uint64_t)g + 1)), kThreads, 0, s>>>(
         ul, row_off, row_job, nrows, xprefix, d_xoffs, g, ctx->d_flag, d_jo);
@@ -1240,7 +1258,11 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         const cudaStream_t sc = (ci & 1) ? sa : s;
         unsigned int *counter = ctx->d_flag + ((ci & 1) && sa != s ? 5 : 1);
         AccArgs b = aa;
-        b.work_counter = counter;
+        // the first chunk has counters of its own, cleared with the rest
+        const auto next_counter = [&](int k) {
+            b.work_counter = ci == 0 ? work + 3 + k : counter;
+            if (ci) GS_CUDA(cudaMemsetAsync(counter, 0, 4, sc));
+        };
         b.chunk_base = c.first;
         b.out_keys = out_k[bi];
         b.out_vals = out_v[bi];
@@ -1249,7 +1271,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         b.nunits = (uint32_t)nu;
         b.l0 = (uint32_t)c.lu0;
         b.l1 = (uint32_t)c.lu1;
-        GS_CUDA(cudaMemsetAsync(counter, 0, 4, sc));
+        next_counter(0);
         GS_CUDA(cudaEventRecord(kev[2 * ci], sc));
         if (light_once) {
             launch_light_copy(b, ctx->sm_count, sc);
@@ -1259,13 +1281,13 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         b.units = Hchunk + c.h0;
         b.nunits = (uint32_t)(c.h1 - c.h0);
         if (nh > nnarrow) {
-            GS_CUDA(cudaMemsetAsync(counter, 0, 4, sc));
+            next_counter(1);
             launch_heavy(b, true, (int)std::min<uint64_t>(gh, std::max<uint64_t>(1, b.nunits)), sc);
         }
         if (nnarrow) {
             b.unit_off += c.h0;
             b.part_off += c.h0;
-            GS_CUDA(cudaMemsetAsync(counter, 0, 4, sc));
+            next_counter(2);
             launch_narrow(b, true, ctx->sm_count, sc);
         }
         b.units = SR.get() + c.s0;
@@ -1300,11 +1322,6 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
                 deliver_slice(J.sink, k2, out_v[bi].get() + (a0 - c0), a1 - a0, a0 - job_first[j], job_nnz[j],
                               s2, J.stats, bst.bytes_d2h, 2);
                 continue;
-            }
-            if (G[j]->wide) {
-                // relabeled output keys back to x_f << Y_nfbits | y_f
-                wide_remap_keys(*G[j]->wide, out_k[bi].get() + (a0 - c0), a1 - a0, s2);
-                GS_CUDA(cudaStreamSynchronize(s2));
             }
             deliver_slice(J.sink, out_k[bi].get() + (a0 - c0), out_v[bi].get() + (a0 - c0), a1 - a0,
                           a0 - job_first[j], job_nnz[j], s2, J.stats, bst.bytes_d2h);
@@ -1663,7 +1680,7 @@ void plan_execute(gsparc_plan *P, uint64_t chunk, uint64_t *keys, float *vals, u
     b.sprefix = gp.sprefix.get() + c.s0;
     launch_stream(b, gp.gs_grid, s);
     for (int j = 0; j < gp.g; ++j) {
-        if (!gp.jobs[j]->wide) continue;
+        if (!gp.jobs[j]->wide || gp.jobs[j]->key_words == 1) continue;  // written with final keys
         const uint64_t a0 = std::max(c.first, gp.job_first[j]), a1 = std::min(c.first + c.n, gp.job_first[j + 1]);
         if (a1 > a0) wide_remap_keys(*gp.jobs[j]->wide, keys + (a0 - c.first), a1 - a0, s);
     }

@@ -70,6 +70,7 @@ struct BatchJob {
     int y_nfbits;       // the job's Y free bits (output key = x_f << y_nfbits | y_f)
     uint32_t ncols;     // the job's distinct Y free indices
     uint32_t ydup;      // nonzero: the job's Y repeats a coordinate
+    uint32_t wide;      // nonzero: relabeled, with cols and y_nfbits of the original operands
     uint64_t cols_off;  // where the job's distinct Y free indices start in `cols`
 };
 
@@ -89,8 +90,9 @@ struct AccArgs {
     // Y side
     const uint32_t *yrank;
     const float *yval;
-    const uint64_t *ykeys;     // sorted Y keys (c << nfbits | y_f, job id above): y_f without the column table
+    const uint64_t *ykeys;     // sorted Y keys (c << nfbits | y_f, job id above): y_f without the column table (not of wide jobs)
     const uint64_t *cols;
+    int any_wide;              // some job is wide (BatchJob)
     int y_nfbits;
     // single-run rows (stream path): the matched X nonzero of every such row,
     // and the product prefix over the listed rows (nunits + 1 entries)

@@ -34,6 +34,22 @@ inline int grid_for(uint64_t n) {
 __device__ __forceinline__ uint64_t shr(uint64_t v, int s) { return s >= 64 ? 0ull : (v >> s); }
 __device__ __forceinline__ uint64_t low_mask(int b) { return b >= 64 ? ~0ull : ((1ull << b) - 1); }
 
+// A thread's 8 consecutive items move as 16-byte words where all are there
+// (arrays are 256-byte aligned, so items 8 t of 4 and 8 bytes are aligned).
+__device__ __forceinline__ void load8(const uint32_t *p, uint32_t (&v)[kScanItems]) {
+    const uint4 a = *reinterpret_cast<const uint4 *>(p), b = *reinterpret_cast<const uint4 *>(p + 4);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+
+__device__ __forceinline__ void load8(const uint64_t *p, uint64_t (&v)[kScanItems]) {
+#pragma unroll
+    for (int q = 0; q < kScanItems; q += 2) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(p + q);
+        v[q] = a.x;
+        v[q + 1] = a.y;
+    }
+}
+
 // Y: runs of (job, contract key).  A job whose Y repeats a coordinate gets
 // ydup[job] set: its runs may hold a free index twice, so none of its rows is
 // streamed.
@@ -56,12 +72,15 @@ __global__ void __launch_bounds__(kScanThreads)
     }
     uint64_t last_word = ~0ull;
     uint32_t word = 0;
+    uint64_t kk[kScanItems];
+    const bool whole = i0 + kScanItems <= ny;
+    if (whole) load8(ykeys + i0, kk);
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) {
         const uint64_t i = i0 + q;
         rk[q] = 0;
         if (i < ny) {
-            const uint64_t key = ykeys[i];
+            const uint64_t key = whole ? kk[q] : ykeys[i];
             const uint64_t j = shr(key, kby);
             const BPrep b = jobs[j];
             const uint64_t loc = key & km;
@@ -178,6 +197,7 @@ __global__ void k_y_ranks(const uint64_t *__restrict__ ykeys, uint64_t ny, int k
         BatchJob b;
         b.y_nfbits = jobs[j].y_nfbits;
         b.ydup = ydup[j];
+        b.wide = 0;
         b.cols_off = wpre[jobs[j].col_word0];
         b.ncols = (uint32_t)((j + 1 < (uint64_t)g ? wpre[jobs[j + 1].col_word0] : cnts[kCntCols]) - b.cols_off);
         acc[j] = b;
@@ -194,11 +214,17 @@ __global__ void __launch_bounds__(kScanThreads)
     uint32_t c[kScanItems];
     uint32_t flags = 0;
     uint64_t x[2] = {0, 0};  // products; matched nonzeros and (above 32 bits) rows
+    const bool whole = i0 + kScanItems <= nx;
+    uint64_t fl = 0;  // 8 flag bytes
+    if (whole) {
+        load8(cnt + i0, c);
+        fl = *reinterpret_cast<const uint64_t *>(row_flag + i0);
+    }
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) {
         const uint64_t i = i0 + q;
-        c[q] = i < nx ? cnt[i] : 0u;
-        if (i < nx && row_flag[i]) flags |= 1u << q;
+        if (!whole) c[q] = i < nx ? cnt[i] : 0u;
+        if (whole ? (fl >> (8 * q) & 0xffu) != 0 : i < nx && row_flag[i]) flags |= 1u << q;
         x[0] += c[q];
         x[1] += (c[q] != 0) + ((uint64_t)(flags >> q & 1u) << 32);
     }
@@ -206,6 +232,21 @@ __global__ void __launch_bounds__(kScanThreads)
     uint32_t m = (uint32_t)x[1], row = (uint32_t)(x[1] >> 32);  // rows that start before this nonzero
     uint64_t p = x[0];
     const uint64_t km = low_mask(kbx);
+    if (whole) {
+        uint64_t pp[kScanItems];
+        uint32_t mm[kScanItems];
+#pragma unroll
+        for (int q = 0; q < kScanItems; ++q) {
+            pp[q] = q ? pp[q - 1] + c[q - 1] : p;
+            mm[q] = q ? mm[q - 1] + (c[q - 1] != 0) : m;
+        }
+#pragma unroll
+        for (int q = 0; q < kScanItems; q += 2)
+            *reinterpret_cast<ulonglong2 *>(r.xprefix + i0 + q) = make_ulonglong2(pp[q], pp[q + 1]);
+#pragma unroll
+        for (int q = 0; q < kScanItems; q += 4)
+            *reinterpret_cast<uint4 *>(r.mpre + i0 + q) = make_uint4(mm[q], mm[q + 1], mm[q + 2], mm[q + 3]);
+    }
 #pragma unroll
     for (int q = 0; q < kScanItems; ++q) {
         const uint64_t i = i0 + q;
@@ -219,8 +260,10 @@ __global__ void __launch_bounds__(kScanThreads)
             r.row_job[row] = (uint16_t)j;
             ++row;
         }
-        r.xprefix[i] = p;
-        r.mpre[i] = m;
+        if (!whole) {
+            r.xprefix[i] = p;
+            r.mpre[i] = m;
+        }
         if (c[q]) {
             r.mrun[m] = (uint32_t)i;
             r.mrow[m] = row - 1;
@@ -237,6 +280,41 @@ __global__ void __launch_bounds__(kScanThreads)
         cnts[kCntRows] = nr;
         cnts[kCntProducts] = sh.through[0];
     }
+}
+
+// Relabeled jobs whose output keys fit 64 bits: the tables that output keys are
+// made from (row_xf, cols, the job's Y free bits) get the original values, so
+// every kernel writes final keys.  As a pass over the finished output the same
+// map took 199 us for 6.2e7 outputs of 4e5 x 2.5e5 nonzeros.
+__global__ void k_wide_tables(const WideTab *__restrict__ tab, int g, const uint16_t *__restrict__ row_job,
+                              uint64_t *__restrict__ row_xf, uint64_t *__restrict__ cols,
+                              BatchJob *__restrict__ acc, const uint64_t *__restrict__ cnts,
+                              const unsigned int *__restrict__ err) {
+    if (*err & kScanErr) return;
+    const uint64_t nr = cnts[kCntRows], nc = cnts[kCntCols];
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint64_t r = t0; r < nr; r += stride) {
+        const WideTab t = tab[row_job[r]];
+        if (t.xf) row_xf[r] = t.xf[row_xf[r]];
+    }
+    for (uint64_t c = t0; c < nc; c += stride) {
+        int lo = 0, hi = g;  // last job whose columns start at or before c
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (acc[mid].cols_off <= c)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        const WideTab t = tab[lo];
+        if (t.xf) cols[c] = t.yf[cols[c]];
+    }
+    for (uint64_t j = t0; j < (uint64_t)g; j += stride)
+        if (tab[j].xf) {
+            acc[j].y_nfbits = tab[j].nfbits_y;
+            acc[j].wide = 1;
+        }
 }
 
 // Row classes: single-run rows of jobs without repeated Y coordinates stream
@@ -285,6 +363,10 @@ __global__ void __launch_bounds__(kScanThreads)
             }
             r.row_prod[i] = pr[q];
             r.row_class[i] = cl[q];
+            if (cl[q] == kRowHeavy && r.row_rb) {
+                r.row_rb[i] = 0xffffffffu;
+                r.row_mx[i] = 0u;
+            }
             r.row_nnz[i] = cl[q] == kRowStream ? (uint32_t)pr[q] : 0u;
             x[0] += (cl[q] >= kRowHeavy) + ((uint64_t)(cl[q] == kRowStream) << 32);
             x[1] += (cl[q] == kRowLight) + ((uint64_t)(cl[q] == kRowNarrow) << 32);
@@ -374,9 +456,9 @@ __global__ void __launch_bounds__(kScanThreads)
 // 5e4 runs took 1155 us (200 warps at work); now 146.
 __global__ void k_matched_runs(const uint32_t *__restrict__ pos, const uint32_t *__restrict__ cnt,
                                const uint32_t *__restrict__ yrank, RowArrays r, const uint64_t *__restrict__ cnts,
-                               uint32_t *__restrict__ row_rb, uint32_t *__restrict__ row_mx,
                                const unsigned int *__restrict__ err) {
     if (*err & kScanErr) return;
+    uint32_t *const row_rb = r.row_rb, *const row_mx = r.row_mx;
     const uint64_t n = r.row_k0[cnts[kCntRows]];  // matched nonzeros
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -415,8 +497,7 @@ __global__ void k_matched_runs(const uint32_t *__restrict__ pos, const uint32_t 
 }
 
 __global__ void __launch_bounds__(kScanThreads)
-    k_heavy_words(RowArrays r, const uint32_t *__restrict__ row_rb, const uint32_t *__restrict__ row_mx,
-                  uint32_t *__restrict__ w_all, uint32_t *__restrict__ w_dense, uint64_t *__restrict__ off_all,
+    k_heavy_words(RowArrays r, uint32_t *__restrict__ w_all, uint32_t *__restrict__ w_dense, uint64_t *__restrict__ off_all,
                   uint64_t *__restrict__ off_dense, uint64_t *__restrict__ cnts, ScanState st) {
     __shared__ ScanShared<2> sh;
     if (ld_acquire(st.err) & kScanErr) return;
@@ -431,7 +512,7 @@ __global__ void __launch_bounds__(kScanThreads)
         wa[q] = wd[q] = 0;
         if (i0 + q < n) {
             const uint32_t row = r.H[i0 + q];
-            const uint64_t span = (uint64_t)row_mx[row] - row_rb[row] + 1, prod = r.row_prod[row];
+            const uint64_t span = (uint64_t)r.row_mx[row] - r.row_rb[row] + 1, prod = r.row_prod[row];
             // narrow rows keep no bitmap here
             const uint32_t words = r.row_class[row] == kRowHeavy ? (uint32_t)(((span + 127) >> 7) << 2) : 0u;
             wa[q] = span <= kKeepBitsMax * prod ? words : 0u;
@@ -456,6 +537,30 @@ __global__ void __launch_bounds__(kScanThreads)
         cnts[kCntBmAll] = sh.through[0];
         cnts[kCntBmDense] = sh.through[1];
     }
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+    k_row_offsets(const uint32_t *__restrict__ row_nnz, uint64_t n, uint64_t *__restrict__ row_off, ScanState st) {
+    __shared__ ScanShared<1> sh;
+    const uint32_t tile = next_tile(st, sh);
+    const uint64_t i0 = (uint64_t)tile * kScanTile + (uint64_t)threadIdx.x * kScanItems;
+    uint32_t c[kScanItems];
+    if (i0 + kScanItems <= n)
+        load8(row_nnz + i0, c);
+    else
+#pragma unroll
+        for (int q = 0; q < kScanItems; ++q) c[q] = i0 + q < n ? row_nnz[i0 + q] : 0u;
+    uint64_t x[1] = {0};
+#pragma unroll
+    for (int q = 0; q < kScanItems; ++q) x[0] += c[q];
+    if (!tile_scan<1>(st, sh, tile, x)) return;
+#pragma unroll
+    for (int q = 0; q < kScanItems; ++q)
+        if (i0 + q < n) {
+            row_off[i0 + q] = x[0];
+            x[0] += c[q];
+        }
+    if ((uint64_t)(tile + 1) * kScanTile >= n && threadIdx.x == 0) row_off[n] = sh.through[0];
 }
 
 void launched() {
@@ -496,6 +601,14 @@ void launch_x_rows(const uint64_t *xkeys, uint64_t nx, int kbx, const BPrep *job
     launched();
 }
 
+void launch_wide_tables(const WideTab *tab, int g, uint64_t n, const uint16_t *row_job, uint64_t *row_xf,
+                        uint64_t *cols, BatchJob *acc, const uint64_t *cnts, const unsigned int *err,
+                        cudaStream_t s) {
+    k_wide_tables<<<grid_for(std::max<uint64_t>(n, (uint64_t)g)), kThreads, 0, s>>>(tab, g, row_job, row_xf, cols, acc,
+                                                                                    cnts, err);
+    launched();
+}
+
 void launch_row_classes(uint64_t nx, const BPrep *jobs, const BatchJob *acc, const uint64_t *range,
                         const RowArrays &r, uint64_t *cnts, const ScanState &st, cudaStream_t s) {
     if (nx == 0) return;
@@ -511,19 +624,26 @@ void launch_light_units(uint64_t nx, uint64_t bin, const RowArrays &r, uint64_t 
 }
 
 void launch_matched_runs(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, const uint32_t *yrank,
-                         const RowArrays &r, uint32_t *row_rb, uint32_t *row_mx, const uint64_t *cnts,
-                         const unsigned int *err, cudaStream_t s) {
+                         const RowArrays &r, const uint64_t *cnts, const unsigned int *err, cudaStream_t s) {
     if (nx == 0) return;
-    k_matched_runs<<<grid_for(nx), kThreads, 0, s>>>(pos, cnt, yrank, r, cnts, row_rb, row_mx, err);
+    k_matched_runs<<<grid_for(nx), kThreads, 0, s>>>(pos, cnt, yrank, r, cnts, err);
     launched();
 }
 
-void launch_heavy_bitmaps(uint64_t nx, const RowArrays &r, const uint32_t *row_rb, const uint32_t *row_mx,
-                          uint32_t *w_all, uint32_t *w_dense, uint64_t *off_all, uint64_t *off_dense, uint64_t *cnts,
-                          const ScanState &st, cudaStream_t s) {
+void launch_heavy_bitmaps(uint64_t nx, const RowArrays &r, uint32_t *w_all, uint32_t *w_dense, uint64_t *off_all,
+                          uint64_t *off_dense, uint64_t *cnts, const ScanState &st, cudaStream_t s) {
     if (nx == 0) return;
-    k_heavy_words<<<(unsigned)scan_tiles(nx), kScanThreads, 0, s>>>(r, row_rb, row_mx, w_all, w_dense, off_all,
-                                                                    off_dense, cnts, st);
+    k_heavy_words<<<(unsigned)scan_tiles(nx), kScanThreads, 0, s>>>(r, w_all, w_dense, off_all, off_dense, cnts, st);
+    launched();
+}
+
+void launch_row_offsets(const uint32_t *row_nnz, uint64_t nrows, uint64_t *row_off, const ScanState &st,
+                        cudaStream_t s) {
+    if (nrows == 0) {
+        GS_CUDA(cudaMemsetAsync(row_off, 0, 8, s));
+        return;
+    }
+    k_row_offsets<<<(unsigned)scan_tiles(nrows), kScanThreads, 0, s>>>(row_nnz, nrows, row_off, st);
     launched();
 }
 

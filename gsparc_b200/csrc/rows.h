@@ -76,27 +76,39 @@ struct RowArrays {
     uint32_t *lrun;      // [light runs] their X nonzeros, light row after light row
     uint32_t *lrow;      // [light runs] their light rows (indices into L)
     uint64_t *loff;      // [light runs] products of the light rows' runs before each one
+    uint32_t *row_rb, *row_mx;  // heavy rows: all ones and 0 (null: not wanted)
 };
 // Match of every X nonzero -> prefix sums, matched list and rows.
 void launch_x_rows(const uint64_t *xkeys, uint64_t nx, int kbx, const BPrep *jobs, const uint32_t *cnt,
                    const uint8_t *row_flag, const RowArrays &r, uint64_t *cnts, const ScanState &st, cudaStream_t s);
+// A relabeled job (wide.cu) whose output keys fit 64 bits: rank -> original free
+// part of X and Y, original Y free bits.  xf null: not one.
+struct WideTab {
+    const uint64_t *xf, *yf;
+    int nfbits_y, pad;
+};
+// Maps row_xf, cols and the Y free bits of those jobs (n: the larger of nx, ny).
+void launch_wide_tables(const WideTab *tab, int g, uint64_t n, const uint16_t *row_job, uint64_t *row_xf,
+                        uint64_t *cols, BatchJob *acc, const uint64_t *cnts, const unsigned int *err,
+                        cudaStream_t s);
 // Row classes, their lists and product prefixes (rows outside `range` get no class).
 void launch_row_classes(uint64_t nx, const BPrep *jobs, const BatchJob *acc, const uint64_t *range,
                         const RowArrays &r, uint64_t *cnts, const ScanState &st, cudaStream_t s);
 // Light units: consecutive light rows of fewer than bin + light_max products.
 void launch_light_units(uint64_t nx, uint64_t bin, const RowArrays &r, uint64_t *cnts, const ScanState &st,
                         cudaStream_t s);
-// The light rows' runs (lrun, lrow, loff) and, with row_rb (all ones at entry)
-// and row_mx (zeros), the rank span of every heavy row.
+// The light rows' runs (lrun, lrow, loff) and, with row_rb and row_mx, the rank
+// span of every heavy row.
 void launch_matched_runs(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, const uint32_t *yrank,
-                         const RowArrays &r, uint32_t *row_rb, uint32_t *row_mx, const uint64_t *cnts,
-                         const unsigned int *err, cudaStream_t s);
+                         const RowArrays &r, const uint64_t *cnts, const unsigned int *err, cudaStream_t s);
 // Kept bitmaps: of every heavy row the words with all / only dense
 // rows kept (w_*, by row), their word offsets (off_*, by row) and totals.
-void launch_heavy_bitmaps(uint64_t nx, const RowArrays &r, const uint32_t *row_rb, const uint32_t *row_mx,
-                          uint32_t *w_all, uint32_t *w_dense,
+void launch_heavy_bitmaps(uint64_t nx, const RowArrays &r, uint32_t *w_all, uint32_t *w_dense,
                           uint64_t *off_all, uint64_t *off_dense, uint64_t *cnts, const ScanState &st, cudaStream_t s);
 
+// row_off[r] = outputs before row r (nrows + 1 entries).
+void launch_row_offsets(const uint32_t *row_nnz, uint64_t nrows, uint64_t *row_off, const ScanState &st,
+                        cudaStream_t s);
 // unit_off[0..n] and part_off[0..n) of a heavy list (narrow.cu), units of about
 // `slice` products.
 void launch_narrow_units(const uint32_t *list, uint32_t n, const uint8_t *row_class, const uint64_t *row_prod,

@@ -65,13 +65,18 @@ __device__ __forceinline__ uint64_t low_mask(int b) { return b >= 64 ? ~0ull : (
 constexpr int kRowBatch = 512;  // rows whose parameters are staged at once
 constexpr int SU = 4;           // outputs per thread with loads in flight
 
+// WIDE: the group has relabeled jobs, whose Y keys hold ranks: their rows take
+// the column from the table (a kernel of its own, as the extra shared load an
+// output cost the others 2% of the numeric pass).
+template <bool WIDE>
 __global__ void __launch_bounds__(ST, 6) k_stream(AccArgs a) {
     __shared__ __align__(16) uint16_t s_row[kStreamTile];  // staged row of every output of the tile
     __shared__ uint32_t s_tmp[33];
     __shared__ uint64_t s_pre[kRowBatch + 1];  // flat start of every staged row (+ the end)
     __shared__ uint64_t s_xf[kRowBatch];       // x_f << Y_nfbits
     __shared__ uint64_t s_o0[kRowBatch];       // row's first slot in the chunk buffer
-    __shared__ uint64_t s_ym[kRowBatch];       // mask of the y_f bits of a Y key
+    __shared__ uint64_t s_ym[kRowBatch];       // mask of the y_f bits of a Y key (WIDE, 0: the table is read)
+    __shared__ uint64_t s_co[WIDE ? kRowBatch : 1];  // the job's columns in the table
     __shared__ uint32_t s_j0[kRowBatch];       // row's first Y entry
     __shared__ float s_xv[kRowBatch];          // the row's X value
     __shared__ uint64_t s_k[2];
@@ -107,6 +112,11 @@ __global__ void __launch_bounds__(ST, 6) k_stream(AccArgs a) {
                 s_xf[i] = shl(a.row_xf[row], y_nfbits);
                 s_o0[i] = a.row_off[row] - a.chunk_base;
                 s_ym[i] = low_mask(y_nfbits);
+                if (WIDE) {
+                    const BatchJob job = a.jobs[a.row_job[row]];
+                    if (job.wide) s_ym[i] = 0ull;
+                    s_co[i] = job.cols_off;
+                }
                 s_j0[i] = a.pos[xi];
                 s_xv[i] = a.xval[xi];
             }
@@ -164,7 +174,12 @@ __global__ void __launch_bounds__(ST, 6) k_stream(AccArgs a) {
                         li[u] = lo;
                         pp[u] = (uint32_t)(t - s_pre[lo]);
                         const uint32_t j = s_j0[lo] + pp[u];
-                        yk[u] = a.ykeys[j];
+                        if (!WIDE) {
+                            yk[u] = a.ykeys[j];
+                        } else {
+                            const uint64_t ym = s_ym[lo];
+                            yk[u] = ym ? a.ykeys[j] & ym : a.cols[s_co[lo] + a.yrank[j]];
+                        }
                         yv[u] = a.yval[j];
                     }
                 }
@@ -175,7 +190,7 @@ __global__ void __launch_bounds__(ST, 6) k_stream(AccArgs a) {
                         const uint32_t i = li[u];
                         const uint64_t o = s_o0[i] + pp[u];
                         if (o < a.out_cap) {
-                            __stcs(a.out_keys + o, (unsigned long long)(s_xf[i] | (yk[u] & s_ym[i])));
+                            __stcs(a.out_keys + o, (unsigned long long)(s_xf[i] | (WIDE ? yk[u] : yk[u] & s_ym[i])));
                             __stcs(a.out_vals + o, s_xv[i] * yv[u]);
                         } else {
                             atomicOr(a.err, 4u);
@@ -192,14 +207,17 @@ __global__ void __launch_bounds__(ST, 6) k_stream(AccArgs a) {
 
 void launch_stream(const AccArgs &a, int grid, cudaStream_t s) {
     if (a.nunits == 0) return;
-    k_stream<<<grid, ST, 0, s>>>(a);
+    if (a.any_wide)
+        k_stream<true><<<grid, ST, 0, s>>>(a);
+    else
+        k_stream<false><<<grid, ST, 0, s>>>(a);
     count_launch();
     GS_CUDA(cudaGetLastError());
 }
 
 int stream_blocks_per_sm() {
     int n = 0;
-    GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_stream, ST, 0));
+    GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_stream<false>, ST, 0));
     return n > 0 ? n : 1;
 }
 

@@ -18,8 +18,10 @@
 // equal contract parts get equal ranks, so X' and Y' match exactly where X and
 // Y do.  Every operand has fewer than 2^31 nonzeros, so F, G < 2^31 and
 // C < 2^32 and the relabeled keys are at most 63 bits wide.  Output keys
-// F << bits(G) | G are mapped back to x_f << Y_nfbits | y_f on every output
-// chunk before it is delivered (order is unchanged by the map).
+// F << bits(G) | G stand for x_f << Y_nfbits | y_f: the planning maps the tables
+// that output keys are made from (k_wide_tables, rows.cu; the order does not
+// change), so the engine writes final keys.  128-bit keys, and a plan's keys
+// over 64 bits, are mapped on every output chunk before it is delivered.
 #include <cub/cub.cuh>
 
 #include "engine.h"
