@@ -435,7 +435,7 @@ struct GroupPlan {
     DBuf<float> xperm, yperm, xvals, yvals;
     DBuf<uint64_t> ykeys;  // sorted Y keys (the single-run-row copy reads y_f from them)
     DBuf<BatchJob> d_acc;
-    DBuf<uint32_t> rank, pos, cnt, mpre, mrun, row_start, L, ustart, lk0, lrun, lrow, H, H2, SR, row_xi, cursor, pend;
+    DBuf<uint32_t> rank, ycol, pos, cnt, mpre, mrun, row_start, L, ustart, lk0, lrun, lrow, H, H2, SR, row_xi, cursor, pend;
     DBuf<uint64_t> cols, xprefix, row_xf, sprefix, row_off, lpre, loff;
     DBuf<uint16_t> row_job;
     DBuf<uint32_t> Hc;         // heavy rows grouped by chunk (several chunks only)
@@ -846,6 +846,18 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     const uint64_t nnarrow = fits(4 * nbm_words + 8 * nparts, 16) ? hc_cnt[kCntNarrow] : 0;
     const uint8_t *narrow_class = nnarrow ? row_class.get() : nullptr;
 
+    // y_f of every Y entry for the heavy rows, where it fits 32 bits and the memory allows
+    DBuf<uint32_t> ycol;
+    {
+        int most = 0;
+        for (Job *q : G)
+            most = std::max(most, q->wide && q->key_words == 1 ? q->wide->nfbits_y : q->LY.nfbits);
+        if (nh > nnarrow && most <= 32 && fits(4 * ny, 16)) {
+            ycol.reset(A, ny, s);
+            launch_y_cols32(ykeys, ny, kby, d_acc, cols, rank, ycol, plan_err, s);
+        }
+    }
+
     // heavy rows largest first (H itself stays in row order for chunk planning)
     DBuf<uint32_t> H2;
     const uint32_t *Hs = H.get();
@@ -907,6 +919,8 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     aa.ykeys = ykeys;
     aa.cols = cols;
     aa.any_wide = any_wide;
+    aa.ycol = ycol.get() ? ycol.get() : rank.get();
+    aa.col_is_key = ycol.get() != nullptr;
     aa.work_counter = ctx->d_flag + 1;
     aa.cursor = cursor;
     aa.pend = pend;
@@ -1134,6 +1148,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         keep->tabs = std::move(tabs);
         keep->d_acc = std::move(d_acc);
         keep->rank = std::move(rank);
+        keep->ycol = std::move(ycol);
         keep->pos = std::move(pos);
         keep->cnt = std::move(cnt);
         keep->mpre = std::move(mpre);

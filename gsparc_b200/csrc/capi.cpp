@@ -136,8 +136,8 @@ gsparc_status gsparc_ctx_set_tiles(gsparc_ctx *ctx, uint64_t light_row_max, uint
         GS_REQUIRE(ctx, GSPARC_EINVAL, "null context");
         GS_REQUIRE(light_row_max <= gs::kLightCap / 2, GSPARC_EINVAL,
                    "light_row_max above " + std::to_string(gs::kLightCap / 2));
-        GS_REQUIRE(heavy_window_cap == 0 || (heavy_window_cap >= 256 && heavy_window_cap <= (uint32_t)gs::kHeavyCap),
-                   GSPARC_EINVAL, "heavy_window_cap must be 0 or 256.." + std::to_string(gs::kHeavyCap));
+        GS_REQUIRE(heavy_window_cap == 0 || (heavy_window_cap >= 256 && heavy_window_cap <= (uint32_t)gs::kHeavyCapMax),
+                   GSPARC_EINVAL, "heavy_window_cap must be 0 or 256.." + std::to_string(gs::kHeavyCapMax));
         ctx->light_row_max = light_row_max;
         ctx->heavy_window_cap = heavy_window_cap;
     });

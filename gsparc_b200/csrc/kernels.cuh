@@ -92,6 +92,8 @@ struct AccArgs {
     const float *yval;
     const uint64_t *ykeys;     // sorted Y keys (c << nfbits | y_f, job id above): y_f without the column table (not of wide jobs)
     const uint64_t *cols;
+    const uint32_t *ycol;      // column of every Y entry: its y_f (col_is_key) or its rank in cols
+    int col_is_key;
     int any_wide;              // some job is wide (BatchJob)
     int y_nfbits;
     // single-run rows (stream path): the matched X nonzero of every such row,
@@ -144,8 +146,9 @@ struct AccArgs {
 
 constexpr int kHeavyThreads = 512;
 constexpr int kHeavyRW = 1 << 17;  // column ranks covered by one window's touched bitmap
-constexpr int kHeavyCap = 8192;    // output slots (compensated accumulators) per window
+constexpr int kHeavyCap = 6656;    // output slots (compensated accumulators, column) per window
                                    // (sized so two CTAs fit one SM's shared memory)
+constexpr int kHeavyCapMax = 8192; // largest window a caller may ask for (kHeavyCap is used above it)
 constexpr int kHeavyMaxRuns = 512;   // runs flattened per batch
 constexpr int kGallopWarpRuns = 64;  // up to this many runs per batch: one warp per run search
 constexpr int kLightCap = 4096;    // on-chip ESC capacity (products per unit); half of it for rows of up to kLightRowMax

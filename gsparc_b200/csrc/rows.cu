@@ -317,6 +317,16 @@ __global__ void k_wide_tables(const WideTab *__restrict__ tab, int g, const uint
         }
 }
 
+// y_f of every Y entry in 32 bits (all jobs' Y free bits fit).
+__global__ void k_y_cols32(const uint64_t *__restrict__ ykeys, uint64_t ny, int kby, const BatchJob *__restrict__ acc,
+                           const uint64_t *__restrict__ cols, const uint32_t *__restrict__ rank,
+                           uint32_t *__restrict__ out, const unsigned int *__restrict__ err) {
+    if (*err & kScanErr) return;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ny; i += stride)
+        out[i] = (uint32_t)cols[acc[shr(ykeys[i], kby)].cols_off + rank[i]];
+}
+
 // Row classes: single-run rows of jobs without repeated Y coordinates stream
 // (their output count is their product count), other rows with more than the
 // job's light limit of products are heavy (narrow where the job has few
@@ -598,6 +608,13 @@ void launch_x_rows(const uint64_t *xkeys, uint64_t nx, int kbx, const BPrep *job
                    const uint8_t *row_flag, const RowArrays &r, uint64_t *cnts, const ScanState &st, cudaStream_t s) {
     if (nx == 0) return;
     k_x_rows<<<(unsigned)scan_tiles(nx), kScanThreads, 0, s>>>(xkeys, nx, kbx, jobs, cnt, row_flag, r, cnts, st);
+    launched();
+}
+
+void launch_y_cols32(const uint64_t *ykeys, uint64_t ny, int kby, const BatchJob *acc, const uint64_t *cols,
+                     const uint32_t *rank, uint32_t *out, const unsigned int *err, cudaStream_t s) {
+    if (ny == 0) return;
+    k_y_cols32<<<grid_for(ny), kThreads, 0, s>>>(ykeys, ny, kby, acc, cols, rank, out, err);
     launched();
 }
 

@@ -91,6 +91,9 @@ struct WideTab {
 void launch_wide_tables(const WideTab *tab, int g, uint64_t n, const uint16_t *row_job, uint64_t *row_xf,
                         uint64_t *cols, BatchJob *acc, const uint64_t *cnts, const unsigned int *err,
                         cudaStream_t s);
+// y_f of every Y entry (all jobs' Y free bits fit 32; after launch_wide_tables).
+void launch_y_cols32(const uint64_t *ykeys, uint64_t ny, int kby, const BatchJob *acc, const uint64_t *cols,
+                     const uint32_t *rank, uint32_t *out, const unsigned int *err, cudaStream_t s);
 // Row classes, their lists and product prefixes (rows outside `range` get no class).
 void launch_row_classes(uint64_t nx, const BPrep *jobs, const BatchJob *acc, const uint64_t *range,
                         const RowArrays &r, uint64_t *cnts, const ScanState &st, cudaStream_t s);

@@ -18,8 +18,8 @@
 //     the hardware add returns the old value, from which TwoSum rebuilds the
 //     exact rounding error of that add; errors (and the product's own fma
 //     error) accumulate in a second word;
-//  4. (numeric) a slot -> column table is built from the bitmap (a thread per
-//     word), then every warp writes 32 consecutive slots per step.
+//  4. (numeric) every warp writes 32 consecutive slots per step; the slots'
+//     columns were left there by the products.
 //
 // The window width adapts to the row's density: each window aims at fifteen
 // sixteenths of kHeavyCap outputs at the density of the window before it (at
@@ -56,12 +56,9 @@ constexpr int NWORDS = RW / 32;
 constexpr int CAP = kHeavyCap;
 constexpr int MAXR = kHeavyMaxRuns;
 // Numeric pass, words of the bitmap region: the bitmap (NWORDS words), then
-// the word prefix (16-bit for a kept row's window, whose prefixes past the
-// capacity are clamped, 32-bit for a marked window); step 4 then reuses the
-// region as the slot -> column table (CAP words).
-constexpr int AW = (2 * NWORDS > CAP ? 2 * NWORDS : CAP);
-static_assert(CAP < 65535, "kept windows hold 16-bit prefixes");
-constexpr int WPT_MAX = (NWORDS + T - 1) / T;
+// the word prefix (16 bits, prefixes past the capacity clamped).
+constexpr int AW = NWORDS + NWORDS / 2;
+static_assert(CAP < 65535, "16-bit prefixes");
 constexpr int RW_SYM = 262144;              // symbolic windows: no accumulators or word prefix kept
 constexpr int NWORDS_SYM = RW_SYM / 32;
 constexpr uint32_t INF = 0xffffffffu;
@@ -210,9 +207,9 @@ __device__ __forceinline__ uint32_t compact_parts(uint32_t nb, uint32_t *seg_sta
 // entry by binary search over the part offsets and then only moves forward:
 // it advances to the next part whenever its entry passes the current part's
 // end, so mapping an entry to (part, index) costs a compare and an add.
-constexpr int ILP = 4;
-
-template <class Item, class Load, class Body>
+// ILP: 4 for the symbolic pass; 2 for the numeric one, which spills at 4 (40 B
+// at its limit of 64 registers: numeric pass 10.2 ms against 9.6 for 7.8e5 nonzeros).
+template <int ILP, class Item, class Load, class Body>
 __device__ __forceinline__ void flat_for(const uint32_t *seg_start, const uint32_t *seg_off, uint32_t ns,
                                          Load &&load, Body &&body) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -266,7 +263,7 @@ struct RankItem {
     uint32_t r;
 };
 struct ProdItem {
-    uint32_t r;
+    uint32_t r, c;
     float xv, yv;
 };
 
@@ -330,45 +327,24 @@ struct RowConst {
     uint32_t rb;            // rank of the kept bitmap's bit 0
 };
 
-// Step 4: slot -> column table from the window's bitmap (nwu words from rank
-// W0 at A, their prefixes at A + NWORDS: 16-bit when P16, else 32-bit; read
-// into registers before the table overwrites the region), then coalesced
-// writes of the window's `outputs` outputs and the reset of their
-// accumulators.  Words go to threads cyclically (word tid + q*T), so a dense
-// stretch of the bitmap spreads over many threads instead of a few.
-template <bool P16>
-__device__ __forceinline__ void write_window(const AccArgs &a, uint32_t *A, float *hi, float *lo, uint32_t nwu,
-                                             uint32_t outputs, uint32_t W0, uint32_t out_pos, const RowConst &rc) {
-    const uint32_t tid = threadIdx.x;
-    uint32_t *ocol = A;
-    const uint16_t *wp16 = reinterpret_cast<const uint16_t *>(A + NWORDS);
-    uint32_t myw[WPT_MAX], myp[WPT_MAX];
-#pragma unroll
-    for (int q = 0; q < WPT_MAX; ++q) {
-        const uint32_t w = tid + (uint32_t)q * T;
-        myw[q] = w < nwu ? A[w] : 0u;
-        myp[q] = w < nwu ? (P16 ? (uint32_t)wp16[w] : A[NWORDS + w]) : 0u;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < WPT_MAX; ++q) {
-        uint32_t bw = myw[q];
-        uint32_t slot = myp[q];
-        const uint32_t cbase = W0 + 32u * (tid + (uint32_t)q * T);
-        while (bw && slot < outputs) {
-            ocol[slot++] = cbase + (uint32_t)(__ffs(bw) - 1);
-            bw &= bw - 1;
-        }
-    }
-    __syncthreads();
+// Step 4: coalesced writes of the window's `outputs` outputs and the reset of
+// their accumulators.  The products left every slot's column in ocol: y_f
+// itself where all jobs' fit 32 bits, else the rank, looked up here.  Against a
+// slot table built from the bitmap and a column lookup an output (16.9 of 43
+// thousand cycles a window of 5,500 outputs, more than the accumulation), and
+// with the next window's words fetched meanwhile, the numeric pass took 9.6
+// instead of 11.9 ms for 7.8e5 nonzeros (1.45e9 products, all rows).
+__device__ __forceinline__ void write_window(const AccArgs &a, const uint32_t *ocol, float *hi, float *lo,
+                                             uint32_t outputs, uint32_t out_pos, const RowConst &rc) {
     // The stores stream past L2 so the output does not evict the Y operand.
     const uint64_t xf_hi = rc.xf_hi;
-    const uint64_t *cols = rc.cols;
-    for (uint32_t q = tid; q < outputs; q += T) {
+    const uint64_t *cols = a.col_is_key ? nullptr : rc.cols;
+    for (uint32_t q = threadIdx.x; q < outputs; q += T) {
         const uint64_t o = (uint64_t)out_pos + q;
         const float v = hi[q] + lo[q];
+        const uint32_t c = ocol[q];
         if (o < a.out_cap) {
-            __stcs(a.out_keys + o, (unsigned long long)(xf_hi | cols[ocol[q]]));
+            __stcs(a.out_keys + o, (unsigned long long)(xf_hi | (cols ? cols[c] : (uint64_t)c)));
             __stcs(a.out_vals + o, v);
         } else {
             atomicOr(a.err, 4u);
@@ -385,8 +361,7 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
     // numeric: region A (AW words, see AW); symbolic: the bitmap alone
     uint32_t *A = reinterpret_cast<uint32_t *>(smem_raw);
     uint32_t *bits = A;                                        // [NWK] bitmap
-    uint32_t *wp = A + NWORDS;                                 // [NWORDS] word prefix (marked windows, numeric)
-    uint16_t *wp16 = reinterpret_cast<uint16_t *>(A + NWORDS); // [NWORDS] word prefix (kept rows, numeric)
+    uint16_t *wp16 = reinterpret_cast<uint16_t *>(A + NWORDS); // [NWORDS] word prefix (numeric)
     uint32_t *seg_start = A + (NUMERIC ? AW : NWK);            // [MAXR]
     uint32_t *seg_off = seg_start + MAXR;                      // [MAXR + 4]
     uint32_t *seg_run = seg_off + MAXR + 4;                    // [MAXR]
@@ -394,6 +369,7 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
     float *seg_xv = reinterpret_cast<float *>(seg_cut + MAXR); // [MAXR]  (numeric) X value of each part
     float *hi = seg_xv + (NUMERIC ? MAXR : 0);                 // [CAP]   (numeric)
     float *lo = hi + CAP;                                      // [CAP]   (numeric)
+    uint32_t *ocol = reinterpret_cast<uint32_t *>(lo + CAP);   // [CAP]   (numeric) column of every slot
     __shared__ uint32_t s_tmp[33];
     __shared__ uint32_t s_unit;
     __shared__ uint32_t s_cut;
@@ -475,6 +451,14 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
             // the ranks below R masked off), so nothing is marked and the window
             // ends exactly after its cap-th column.
             uint32_t R = R0;  // every column below R is written
+            // a window's words, asked for while the window before it is written out
+            const auto load_words = [&](uint32_t from) {
+                const uint32_t wo = ((from - s_rc.rb) >> 7) << 2;
+                if (from == INF || wo >= nwr) return;
+                const uint32_t n = min((uint32_t)NWORDS, nwr - wo) >> 2;
+                for (uint32_t q = tid; q < n; q += T) cp_async16(bits + 4u * q, s_rc.src + wo + 4u * q);
+            };
+            load_words(R);
             for (;;) {
                 const uint32_t rb = s_rc.rb;
                 if (R == INF) break;
@@ -483,11 +467,9 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
                 const uint32_t W0 = rb + 32u * wo;
                 const uint32_t nw = min((uint32_t)NWORDS, nwr - wo);
                 const uint32_t skip = R - W0;  // < 128: ranks [W0, R) of words 0..3 are done
-                __syncthreads();  // the previous window no longer reads bits, prefix, table or s_next
-                for (uint32_t q = tid; q < (nw >> 2); q += T) cp_async16(bits + 4u * q, s_rc.src + wo + 4u * q);
                 cp_async_wait_all();
                 if (tid == 0) s_next = INF;
-                __syncthreads();
+                __syncthreads();  // also: the previous window no longer reads prefix, accumulators or ocol
                 // word prefix: thread t owns wpt consecutive words (4 or 8, read as
                 // 16-byte vectors; thread 0 clears the done ranks of words 0..3
                 // and writes them back before any other thread reads them), the
@@ -541,6 +523,7 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
                 uint32_t R1 = W0 + 32u * nw, outputs = Dw;
                 if (Dw == 0) {  // a gap wider than the window (Dw is the same in every thread)
                     R = R1;
+                    load_words(R);  // every thread has read its words before the scan
                     continue;
                 }
                 __syncthreads();
@@ -561,10 +544,11 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
                     const uint32_t ns = compact_parts(nb, seg_start, seg_off, seg_run, seg_cut, s_tmp);
                     for (uint32_t k = tid; k < ns; k += T) seg_xv[k] = a.xval[seg_run[k]];
                     __syncthreads();
-                    flat_for<ProdItem>(
+                    flat_for<2, ProdItem>(
                         seg_start, seg_off, ns,
                         [&](uint32_t k, uint32_t idx, ProdItem &it) {
                             it.r = a.yrank[idx];
+                            it.c = a.ycol[idx];
                             it.yv = a.yval[idx];
                             it.xv = seg_xv[k];
                         },
@@ -574,6 +558,7 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
                             const uint32_t slot =
                                 w < nw ? wp16[w] + __popc(bits[w] & ((1u << (c & 31)) - 1u)) : outputs;
                             if (slot < outputs) {
+                                ocol[slot] = it.c;
                                 const float pr = it.xv * it.yv;
                                 const float pe = fmaf(it.xv, it.yv, -pr);
                                 const float old = atomicAdd(&hi[slot], pr);
@@ -588,12 +573,14 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
                     for (uint32_t k = tid; k < ns; k += T) a.cursor[seg_run[k]] = seg_cut[k];
                     __syncthreads();
                 }
-                write_window<true>(a, A, hi, lo, nw, outputs, W0, out_pos, s_rc);
+                // the next window starts at the row's next column (skipping a gap; INF: none left)
+                R = max(R1, s_next);
+                load_words(R);
+                write_window(a, ocol, hi, lo, outputs, out_pos, s_rc);
                 if (tid == 0) atomicAdd(a.err + 2, 1u);  // windows swept (statistics)
                 out_pos += outputs;
                 row_total += outputs;
-                // the next window starts at the row's next column (skipping a gap; INF: none left)
-                R = max(R1, s_next);
+                __syncthreads();  // s_next is read; the accumulators are clear
             }
             R0 = INF;  // the row is done
         }
@@ -607,7 +594,7 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
             uint32_t ns = 0;
             uint32_t newcols = 0;  // symbolic: columns in this thread's words of the window
             if (NUMERIC) {
-                // the region held the previous window's table (or a kept row's pairs): clear the bitmap
+                // the region held the previous window's bitmap (or a kept row's): clear it
                 __syncthreads();
                 for (uint32_t w = 4u * tid; w < (uint32_t)NWORDS; w += 4u * T)
                     *reinterpret_cast<uint4 *>(bits + w) = make_uint4(0u, 0u, 0u, 0u);
@@ -622,7 +609,7 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
                 ns = compact_parts(nb, seg_start, seg_off, seg_run, seg_cut, s_tmp);
                 if (NUMERIC)
                     for (uint32_t k = tid; k < ns; k += T) seg_xv[k] = a.xval[seg_run[k]];
-                flat_for<RankItem>(
+                flat_for<4, RankItem>(
                     seg_start, seg_off, ns,
                     [&](uint32_t, uint32_t idx, RankItem &it) { it.r = a.yrank[idx]; },
                     [&](uint32_t, uint32_t, const RankItem &it) {
@@ -670,7 +657,7 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
             uint32_t Dw;
             uint32_t run = block_excl_scan_u32<T>(loc, s_tmp, &Dw);
             for (uint32_t w = w0; w < w1; ++w) {
-                wp[w] = run;
+                wp16[w] = (uint16_t)min(run, 0xffffu);
                 run += __popc(bits[w]);
             }
 
@@ -679,7 +666,7 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
             uint32_t R1 = lim, outputs = Dw;
             if (over) {
                 for (uint32_t w = w0; w < w1; ++w) {
-                    const uint32_t pw = wp[w];
+                    const uint32_t pw = wp16[w];  // not clamped at the cut
                     if (pw <= cap && cap < pw + __popc(bits[w])) {
                         const uint32_t b = __fns(bits[w], 0u, (int)(cap - pw + 1));
                         s_cut = R0 + 32u * w + b;
@@ -709,10 +696,11 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
                     for (uint32_t k = tid; k < ns; k += T) seg_xv[k] = a.xval[seg_run[k]];
                     __syncthreads();
                 }
-                flat_for<ProdItem>(
+                flat_for<2, ProdItem>(
                     seg_start, seg_off, ns,
                     [&](uint32_t k, uint32_t idx, ProdItem &it) {
                         it.r = a.yrank[idx];
+                        it.c = a.ycol[idx];
                         it.yv = a.yval[idx];
                         it.xv = seg_xv[k];
                     },
@@ -720,7 +708,8 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
                         if (it.r < R1) {
                             const uint32_t c = it.r - R0;
                             const uint32_t w = c >> 5;
-                            const uint32_t slot = wp[w] + __popc(bits[w] & ((1u << (c & 31)) - 1u));
+                            const uint32_t slot = wp16[w] + __popc(bits[w] & ((1u << (c & 31)) - 1u));
+                            ocol[slot] = it.c;
                             const float pr = it.xv * it.yv;
                             const float pe = fmaf(it.xv, it.yv, -pr);
                             const float old = atomicAdd(&hi[slot], pr);
@@ -736,8 +725,8 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
                 __syncthreads();
             }
 
-            // ---- 4: slot -> column table, then coalesced writes of the window
-            write_window<false>(a, A, hi, lo, nwu, outputs, R0, out_pos, s_rc);
+            // ---- 4: coalesced writes of the window
+            write_window(a, ocol, hi, lo, outputs, out_pos, s_rc);
             if (tid == 0) atomicAdd(a.err + 2, 1u);  // windows swept (statistics)
             out_pos += outputs;
             row_total += outputs;
@@ -762,7 +751,7 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
 
 size_t rowwin_smem(bool numeric) {
     const size_t words = (numeric ? (size_t)AW + MAXR : (size_t)NWORDS_SYM) + MAXR + (MAXR + 4) + MAXR + MAXR;
-    return words * 4 + (numeric ? (size_t)CAP * 8 : 0);
+    return words * 4 + (numeric ? (size_t)CAP * 12 : 0);
 }
 
 }  // namespace
