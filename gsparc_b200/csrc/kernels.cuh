@@ -146,7 +146,7 @@ struct AccArgs {
 
 constexpr int kHeavyThreads = 512;
 constexpr int kHeavyRW = 1 << 17;  // column ranks covered by one window's touched bitmap
-constexpr int kHeavyCap = 6656;    // output slots (compensated accumulators, column) per window
+constexpr int kHeavyCap = 6528;    // output slots (compensated accumulators, column) per window
                                    // (sized so two CTAs fit one SM's shared memory)
 constexpr int kHeavyCapMax = 8192; // largest window a caller may ask for (kHeavyCap is used above it)
 constexpr int kHeavyMaxRuns = 512;   // runs flattened per batch

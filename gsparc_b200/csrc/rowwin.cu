@@ -39,7 +39,13 @@
 // meanwhile), takes the word prefix, ends exactly where the kHeavyCap-th
 // column is passed, and finds every run's part with that end, so windows are
 // full and no product is read twice; the next window starts at the row's next
-// column, so gaps are skipped.
+// column, so gaps are skipped.  A row whose runs fit one batch keeps their
+// cursors, ends and X values in shared memory for all its windows (read from
+// memory they cost each window three dependent loads before its search; a
+// window of a 3.1e5 x 3.1e5 contraction holds about 30 runs and spends a sixth
+// of its time there): numeric passes of 3.1e5 nonzeros 1.99 -> 1.93 ms, of
+// 7.75e5 9.6 -> 9.3 ms.  More shared memory a run means fewer outputs a window
+// (6528 instead of 6656), and two CTAs still fit one SM.
 #include "blockops.cuh"
 #include "kernels.cuh"
 #include "rows.h"
@@ -193,6 +199,131 @@ __device__ __forceinline__ uint32_t compact_parts(uint32_t nb, uint32_t *seg_sta
     const uint32_t at = block_excl_scan_u32<T>(f0 + f1, s_tmp, &ns);  // all reads done before it returns
     if (f0) { seg_start[at] = s0; seg_off[at] = l0; seg_run[at] = r0; seg_cut[at] = c0; }
     if (f1) { seg_start[at + f0] = s1; seg_off[at + f0] = l1; seg_run[at + f0] = r1; seg_cut[at + f0] = c1; }
+    __syncthreads();
+    block_scan_inplace(seg_off, ns, s_tmp);
+    return ns;
+}
+
+// Step A of a kept row whose runs' cursors (cut), ends and X values are in
+// shared memory: the part of every run up to lim, the cursors moved.  Up to
+// kGallopWarpRuns runs: a warp searches two at a time (their loads in flight
+// together), 32 probes 32 entries apart and then the 32 entries before the
+// first one past lim; a part of more than 1024 entries goes on by warp_gallop.
+__device__ __forceinline__ uint32_t find_own_parts(const uint32_t *__restrict__ rank, uint32_t nb, uint32_t lim,
+                                                   uint32_t *seg_start, uint32_t *seg_off, uint32_t *cut,
+                                                   const uint32_t *end) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t nextmin = INF;
+    if (nb <= (uint32_t)kGallopWarpRuns) {
+        for (uint32_t k = warp; k < nb; k += 2 * NWARPS) {
+            uint32_t p[2], e[2], base[2], r[2], hit[2];
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const uint32_t kt = k + t * NWARPS;
+                p[t] = kt < nb ? cut[kt] : 0u;
+                e[t] = kt < nb ? end[kt] : 0u;
+                const uint64_t q = (uint64_t)p[t] + 32u * (lane + 1u) - 1u;
+                r[t] = q < e[t] ? rank[q] : INF;
+            }
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                hit[t] = __ballot_sync(FULL, r[t] >= lim);
+                base[t] = p[t] + 32u * (hit[t] ? __ffs(hit[t]) - 1u : 0u);
+                const uint64_t q = (uint64_t)base[t] + lane;
+                r[t] = hit[t] && q < e[t] ? rank[q] : INF;
+            }
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const uint32_t at = __ffs(__ballot_sync(FULL, r[t] >= lim)) - 1u;
+                uint32_t fr = __shfl_sync(FULL, r[t], at);
+                uint32_t pe = min(base[t] + at, e[t]);
+                if (!hit[t]) pe = warp_gallop(rank, p[t] + 1024u, e[t], lim, &fr);  // all before are below lim
+                const uint32_t kt = k + t * NWARPS;
+                if (kt < nb) {
+                    if (lane == 0) {
+                        seg_start[kt] = p[t];
+                        seg_off[kt] = pe - p[t];
+                        cut[kt] = pe;
+                    }
+                    nextmin = min(nextmin, fr);
+                }
+            }
+        }
+    } else {
+        for (uint32_t k = tid; k < nb; k += T) {
+            const uint32_t p = cut[k], e = end[k];
+            uint32_t pe = p, fr = INF;
+            if (p < e) pe = thread_gallop(rank, p, e, lim, &fr);
+            seg_start[k] = p;
+            seg_off[k] = pe - p;
+            cut[k] = pe;
+            nextmin = min(nextmin, fr);
+        }
+    }
+    return nextmin;
+}
+
+// compact_parts for such rows: the parts' X values (by run in rxv) go along to xv.
+__device__ __forceinline__ uint32_t compact_own_parts(uint32_t nb, uint32_t *seg_start, uint32_t *seg_off,
+                                                      const float *rxv, float *xv, uint32_t *s_tmp) {
+    if (nb <= 64u) {
+        // warp 0 alone, two parts a lane
+        if (threadIdx.x < 32) {
+            const uint32_t k = threadIdx.x;
+            uint32_t st[2], len[2], at[2], off[2];
+            float v[2];
+            uint32_t ns = 0, tot = 0;
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const uint32_t i = k + 32u * t;
+                st[t] = len[t] = 0;
+                v[t] = 0.f;
+                if (i < nb) {
+                    st[t] = seg_start[i];
+                    len[t] = seg_off[i];
+                    v[t] = rxv[i];
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const uint32_t bal = __ballot_sync(FULL, len[t] != 0u);
+                uint32_t x = len[t];
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(FULL, x, o);
+                    if (k >= (uint32_t)o) x += y;
+                }
+                at[t] = ns + __popc(bal & ((1u << k) - 1u));
+                off[t] = tot + x - len[t];
+                ns += __popc(bal);
+                tot += __shfl_sync(FULL, x, 31);
+            }
+            __syncwarp();  // every part was read
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+                if (len[t]) {
+                    seg_start[at[t]] = st[t];
+                    seg_off[at[t]] = off[t];
+                    xv[at[t]] = v[t];
+                }
+            __syncwarp();
+            if (k == 0) {
+                seg_off[ns] = tot;
+                s_tmp[32] = ns;
+            }
+        }
+        __syncthreads();
+        return s_tmp[32];
+    }
+    const uint32_t k0 = 2u * threadIdx.x, k1 = k0 + 1u;
+    uint32_t s0 = 0, l0 = 0, s1 = 0, l1 = 0;
+    if (k0 < nb) { s0 = seg_start[k0]; l0 = seg_off[k0]; }
+    if (k1 < nb) { s1 = seg_start[k1]; l1 = seg_off[k1]; }
+    const uint32_t f0 = l0 ? 1u : 0u, f1 = l1 ? 1u : 0u;
+    uint32_t ns;
+    const uint32_t at = block_excl_scan_u32<T>(f0 + f1, s_tmp, &ns);  // all reads done before it returns
+    if (f0) { seg_start[at] = s0; seg_off[at] = l0; xv[at] = rxv[k0]; }
+    if (f1) { seg_start[at + f0] = s1; seg_off[at + f0] = l1; xv[at + f0] = rxv[k1]; }
     __syncthreads();
     block_scan_inplace(seg_off, ns, s_tmp);
     return ns;
@@ -367,7 +498,8 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
     uint32_t *seg_run = seg_off + MAXR + 4;                    // [MAXR]
     uint32_t *seg_cut = seg_run + MAXR;                        // [MAXR]
     float *seg_xv = reinterpret_cast<float *>(seg_cut + MAXR); // [MAXR]  (numeric) X value of each part
-    float *hi = seg_xv + (NUMERIC ? MAXR : 0);                 // [CAP]   (numeric)
+    float *run_xv = seg_xv + (NUMERIC ? MAXR : 0);             // [MAXR]  (numeric) X value of each run of a kept row
+    float *hi = run_xv + (NUMERIC ? MAXR : 0);                 // [CAP]   (numeric)
     float *lo = hi + CAP;                                      // [CAP]   (numeric)
     uint32_t *ocol = reinterpret_cast<uint32_t *>(lo + CAP);   // [CAP]   (numeric) column of every slot
     __shared__ uint32_t s_tmp[33];
@@ -420,11 +552,21 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
             }
         }
 
+        const bool one_batch = xe - xs <= (uint32_t)MAXR;  // parts from step A stay in place
+        // a kept row's runs are held in shared memory when one batch takes them:
+        // cursors in seg_cut, ends in seg_run, X values in run_xv
+        const bool own = NUMERIC && nwr && one_batch;
         uint32_t mymin = INF;
         for (uint32_t i = xs + tid; i < xe; i += T) {
-            const uint32_t p = a.pos[i];
-            a.cursor[i] = p;
-            if (a.cnt[i]) mymin = min(mymin, a.yrank[p]);
+            const uint32_t p = a.pos[i], c = a.cnt[i];
+            if (NUMERIC && own) {
+                seg_cut[i - xs] = p;
+                seg_run[i - xs] = p + c;
+                run_xv[i - xs] = a.xval[i];
+            } else {
+                a.cursor[i] = p;
+            }
+            if (c) mymin = min(mymin, a.yrank[p]);
         }
         uint32_t R0 = block_min_u32<T>(mymin, s_tmp);
 
@@ -443,7 +585,6 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
         // the row's first slot in the chunk buffer (a chunk holds fewer than 2^32 outputs)
         uint32_t out_pos = NUMERIC ? (uint32_t)(a.row_off[row] - a.chunk_base) : 0u;
         uint32_t row_total = 0;
-        const bool one_batch = xe - xs <= (uint32_t)MAXR;  // parts from step A stay in place
 
         if (NUMERIC && nwr) {
             // ---- kept bitmap: windows are swept contiguously from the row's
@@ -538,12 +679,19 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
                 }
                 for (uint32_t b0 = xs; b0 < xe; b0 += MAXR) {
                     const uint32_t nb = min((uint32_t)MAXR, xe - b0);
-                    const uint32_t nm = find_parts<0>(a, b0, nb, R1, seg_start, seg_off, seg_run, seg_cut);
-                    if (nm != INF) atomicMin(&s_next, nm);
+                    const uint32_t nm = __reduce_min_sync(
+                        FULL, own ? find_own_parts(a.yrank, nb, R1, seg_start, seg_off, seg_cut, seg_run)
+                                  : find_parts<0>(a, b0, nb, R1, seg_start, seg_off, seg_run, seg_cut));
+                    if ((tid & 31) == 0 && nm != INF) atomicMin(&s_next, nm);
                     __syncthreads();
-                    const uint32_t ns = compact_parts(nb, seg_start, seg_off, seg_run, seg_cut, s_tmp);
-                    for (uint32_t k = tid; k < ns; k += T) seg_xv[k] = a.xval[seg_run[k]];
-                    __syncthreads();
+                    uint32_t ns;
+                    if (own) {
+                        ns = compact_own_parts(nb, seg_start, seg_off, run_xv, seg_xv, s_tmp);
+                    } else {
+                        ns = compact_parts(nb, seg_start, seg_off, seg_run, seg_cut, s_tmp);
+                        for (uint32_t k = tid; k < ns; k += T) seg_xv[k] = a.xval[seg_run[k]];
+                        __syncthreads();
+                    }
                     flat_for<2, ProdItem>(
                         seg_start, seg_off, ns,
                         [&](uint32_t k, uint32_t idx, ProdItem &it) {
@@ -570,8 +718,10 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
                             }
                         });
                     __syncthreads();
-                    for (uint32_t k = tid; k < ns; k += T) a.cursor[seg_run[k]] = seg_cut[k];
-                    __syncthreads();
+                    if (!own) {
+                        for (uint32_t k = tid; k < ns; k += T) a.cursor[seg_run[k]] = seg_cut[k];
+                        __syncthreads();
+                    }
                 }
                 // the next window starts at the row's next column (skipping a gap; INF: none left)
                 R = max(R1, s_next);
@@ -750,7 +900,7 @@ __global__ void __launch_bounds__(T, NUMERIC ? 2 : 3) k_rowwin(AccArgs a) {  // 
 }
 
 size_t rowwin_smem(bool numeric) {
-    const size_t words = (numeric ? (size_t)AW + MAXR : (size_t)NWORDS_SYM) + MAXR + (MAXR + 4) + MAXR + MAXR;
+    const size_t words = (numeric ? (size_t)AW + 2 * MAXR : (size_t)NWORDS_SYM) + MAXR + (MAXR + 4) + MAXR + MAXR;
     return words * 4 + (numeric ? (size_t)CAP * 12 : 0);
 }
 
