@@ -1,26 +1,19 @@
-// accumulate.cu -- symbolic and numeric accumulation of matched products.
+// accumulate.cu -- light rows of the accumulation of matched products.
 //
 // Output row r is one X free index x_f (X is sorted free-major, so its
 // nonzeros are contiguous).  Its products are the Y runs matched by the row's
 // X nonzeros; every Y run is sorted by column (the Y free index, carried as a
-// dense rank among Y's distinct free indices).  Two accumulators:
+// dense rank among Y's distinct free indices).  Rows of few products are done
+// here: units of them are expanded, their sorted runs merged and compressed on
+// chip (expand-sort-compress; reference ESC:
+// include/gsparc/contraction.cuh:100-141,506-537), with a compensated
+// sequential sum per output key.  Longer rows: rowwin.cu (windows of columns)
+// and narrow.cu (few columns); rows of one run: stream.cu.  Sums that are
+// exactly zero stay in the output, as in the reference's ESC
+// (include/gsparc/contraction.cuh:532-537).
 //
-//  * heavy rows (many products): a dense window of kHeavyW columns in shared
-//    memory sweeps the row's column range; each run keeps a cursor, so every
-//    window takes exactly the run entries that fall inside it.  Sums are
-//    compensated: the hardware add returns the old value, from which the exact
-//    rounding error of that addition is rebuilt (TwoSum) and accumulated in a
-//    second word; each product's own rounding error (fma) goes there too.
-//    Touched cells are tracked in a bitmap so exact-zero sums still count
-//    (the reference's ESC keeps them, include/gsparc/contraction.cuh:532-537).
-//  * light rows (few products): units of consecutive rows are expanded, their
-//    sorted runs merged and compressed on chip (expand-sort-compress; reference
-//    ESC: include/gsparc/contraction.cuh:100-141,506-537), with a compensated
-//    sequential sum per output key.
-//
-// Both run twice: a symbolic pass that only counts each row's distinct
-// columns, and a numeric pass that writes each row's sorted output at its
-// final offset.
+// Two passes: a symbolic one that counts each row's distinct columns, and a
+// numeric one that writes each row's sorted output at its final offset.
 #include "blockops.cuh"
 #include "kernels.cuh"
 
