@@ -28,6 +28,7 @@
 #include "engine.h"
 #include "kernels.cuh"
 #include "rows.h"
+#include "runtab.h"
 #include "verify.h"
 #include "wide.h"
 
@@ -201,8 +202,7 @@ __global__ void k_bmatch(const uint64_t *__restrict__ xkeys, uint64_t nx, int kb
         uint64_t r = nr;
         if (ctab) {
             const uint2 t = ctab[b.con_word0 + (c >> 5)];
-            const uint32_t bit = 1u << (c & 31);
-            if (t.x & bit) r = (uint64_t)t.y + __popc(t.x & (bit - 1u));
+            r = run_of_key(t.x, t.y, c, nr);
         } else {
             const uint64_t target = shl(j, kby) | c;
             r = lower_bound_dev<uint64_t>(run_key, 0, nr, target);

@@ -16,6 +16,7 @@
 #include "rows.h"
 
 #include "blockops.cuh"
+#include "runtab.h"
 
 namespace gs {
 
@@ -119,11 +120,12 @@ __global__ void __launch_bounds__(kScanThreads)
             run_start[x[0]] = (uint32_t)(i0 + q);
             if (ctab) {
                 const BPrep b = jobs[shr(rk[q], kby)];
-                // masked: an out-of-range index (its job fails) stays in its job's words
-                const uint64_t c = rk[q] & km & low_mask(b.x_ncbits);
-                uint2 *t = ctab + b.con_word0 + (c >> 5);
-                atomicOr(&t->x, 1u << (c & 31));
-                if (first >> q & 1u) t->y = (uint32_t)x[0];
+                const uint64_t c = rk[q] & km;
+                if (run_in_table(c, b.x_ncbits)) {
+                    uint2 *t = ctab + b.con_word0 + (c >> 5);
+                    atomicOr(&t->x, 1u << (c & 31));
+                    if (first >> q & 1u) t->y = (uint32_t)x[0];
+                }
             }
             ++x[0];
         }
