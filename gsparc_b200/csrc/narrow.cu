@@ -392,11 +392,15 @@ size_t narrow_smem(bool numeric, uint32_t cols) {
     return numeric ? NW * ncp * (sizeof(float2) + 1) : 0;
 }
 
+// The kernel's shared memory limit is the function's, not the launch's: every
+// call sets the same one, the widest job's, so that no thread lowers it between
+// another thread's setting and its launch.
 template <bool NUMERIC>
 int narrow_grid(int sm_count, uint32_t cols) {
     int n = 0;
     const size_t sm = narrow_smem(NUMERIC, cols);
-    GS_CUDA(cudaFuncSetAttribute(k_narrow<NUMERIC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    GS_CUDA(cudaFuncSetAttribute(k_narrow<NUMERIC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)narrow_smem(NUMERIC, kNarrowCols)));
     GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_narrow<NUMERIC>, NT, sm));
     return sm_count * std::max(n, 1);
 }
