@@ -324,6 +324,12 @@ class _Staging:
             self.pinned = False
             lib().gsparc_host_unpin(_p(self.buf))
 
+    def __del__(self):  # dropped without being given back: its pages must not stay registered
+        try:
+            self.release()
+        except Exception:
+            pass
+
 
 class _StagingPool:
     """At most `keep` page-locked staging buffers, kept between calls by their
@@ -826,12 +832,9 @@ def sptc_batch(ctx: Context, jobs, sink: str = "host", max_chunk_nnz: int = 0, s
     n = len(jobs)
     arr = (_Job * max(n, 1))()
     keep = []
-    stg = None
+    stg = cb = None
     cols = []
     if sink == "host":
-        stg = ctx._staging.take(staging)
-        cols = [_Collect(stg) for _ in range(n)]
-
         def _cbh(user, k, v, m, first, on_dev):
             cols[int(user or 0)].add(k, v, m, first)
             return 0
@@ -843,12 +846,8 @@ def sptc_batch(ctx: Context, jobs, sink: str = "host", max_chunk_nnz: int = 0, s
         def _cbd(user, k, v, m, first, on_dev):
             return int(bool(on_chunk(int(user or 0), k, v, m, first)))
         cb = CHUNK_FN(_cbd)
-    elif sink == "discard":
-        cb = None
-    else:
+    elif sink != "discard":
         raise ValueError(f"unknown sink {sink!r}")
-    if cb is not None:
-        keep.append(cb)
     for j, job in enumerate(jobs):
         X, Y, cx, cy = job[:4]
         accum = job[4] if len(job) > 4 else ACCUM_AUTO
@@ -865,17 +864,14 @@ def sptc_batch(ctx: Context, jobs, sink: str = "host", max_chunk_nnz: int = 0, s
         J.cy = c2.ctypes.data
         J.accum = int(accum)
         J.sink.user = j
-        if sink == "host":
-            J.sink.kind = SINK_HOST
-            J.sink.host_keys = stg.kp
-            J.sink.host_vals = stg.vp
-            J.sink.host_capacity = stg.nnz
+        J.sink.kind = {"host": SINK_HOST, "device": SINK_DEVICE, "discard": SINK_DISCARD}[sink]
+        if cb is not None:
             J.sink.on_chunk = cb
-        elif sink == "device":
-            J.sink.kind = SINK_DEVICE
-            J.sink.on_chunk = cb
-        else:
-            J.sink.kind = SINK_DISCARD
+    if sink == "host":  # taken when nothing can raise any more before it is given back
+        stg = ctx._staging.take(staging)
+        cols += [_Collect(stg) for _ in range(n)]
+        for j in range(n):
+            arr[j].sink.host_keys, arr[j].sink.host_vals, arr[j].sink.host_capacity = stg.kp, stg.vp, stg.nnz
     st = Stats()
     try:
         rc = lib().gsparc_sptc_batch(ctx.handle, ctypes.cast(arr, ctypes.c_void_p), n, max_chunk_nnz,

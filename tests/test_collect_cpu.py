@@ -57,3 +57,60 @@ def test_pool():
     pool.close()
     pool.give(pool.take(api.STAGING_NNZ))
     assert not pool._free
+
+
+class _Driver:
+    """Stands in for the library: which buffers are registered, a batch that does nothing."""
+
+    def __init__(self):
+        self.registered = set()
+
+    def gsparc_host_pin(self, p, n):
+        self.registered.add(p.value)
+        return 0
+
+    def gsparc_host_unpin(self, p):
+        self.registered.remove(p.value)
+        return 0
+
+    def gsparc_sptc_batch(self, *a):
+        return 0
+
+
+class _Operand:
+    handle = None
+
+
+class _Ctx:
+    handle = None
+
+    def __init__(self):
+        self._staging = api._StagingPool(2)
+
+
+@pytest.mark.parametrize("bad", [(_Operand, _Operand, [0], [0, 1]), (_Operand, _Operand, [0]),
+                                 (_Operand, None, [0], [0])])
+def test_malformed_job_keeps_the_staging(monkeypatch, bad):
+    drv = _Driver()
+    monkeypatch.setattr(api, "lib", lambda: drv)
+    ctx, good = _Ctx(), (_Operand, _Operand, [0], [0])
+    for _ in range(3):
+        with pytest.raises((ValueError, AttributeError)):
+            api.sptc_batch(ctx, [good, bad])
+    res, _ = api.sptc_batch(ctx, [good])
+    assert res[0].keys.size == 0 and len(drv.registered) == 1 == len(ctx._staging._free)
+    st = ctx._staging.take(api.STAGING_NNZ)
+    assert st.pinned  # the pool still has one to give
+    ctx._staging.give(st)
+    ctx._staging.close()
+    assert not drv.registered
+
+
+def test_dropped_staging_is_unregistered(monkeypatch):
+    drv = _Driver()
+    monkeypatch.setattr(api, "lib", lambda: drv)
+    pool = api._StagingPool(2)
+    st = pool.take(api.STAGING_NNZ)
+    assert drv.registered == {st.buf.ctypes.data}
+    del st
+    assert not drv.registered
