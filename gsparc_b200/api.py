@@ -384,8 +384,8 @@ class _CallerStaging:
 
 class _Collect:
     """Gathers the pieces a HOST sink delivers (in order, through `st`) into
-    result arrays: exactly sized when one piece is all, grown by doubling
-    otherwise."""
+    result arrays: exactly sized when one piece is all, grown by doubling and
+    cut to size at the end otherwise."""
 
     def __init__(self, st: _Staging, kw: int = 1):
         self.st, self.kw, self.n = st, kw, 0
@@ -413,8 +413,10 @@ class _Collect:
     def result(self):
         if self.vals is None:
             return np.zeros((0, 2) if self.kw == 2 else 0, np.uint64), np.zeros(0, np.float32)
-        keys, vals = self.keys[: self.kw * self.n], self.vals[: self.n]
-        return (keys.reshape(-1, 2) if self.kw == 2 else keys), vals
+        # the grown arrays' spare end goes back to the system (nothing else refers to them)
+        self.keys.resize(self.kw * self.n, refcheck=False)
+        self.vals.resize(self.n, refcheck=False)
+        return (self.keys.reshape(-1, 2) if self.kw == 2 else self.keys), self.vals
 
 
 # ------------------------------------------------------------------ engine

@@ -114,3 +114,18 @@ def test_dropped_staging_is_unregistered(monkeypatch):
     assert drv.registered == {st.buf.ctypes.data}
     del st
     assert not drv.registered
+
+
+@pytest.mark.parametrize("kw", [1, 2])
+@pytest.mark.parametrize("pieces", [[8], [8, 1], [8] * 5 + [3], [8] * 300 + [1]])
+def test_results_hold_no_spare_memory(kw, pieces):
+    st = _Plain(kw * 8)
+    col = api._Collect(st, kw)
+    for k, n in enumerate(pieces):
+        st.keys[:], st.vals[:] = k, k
+        col.add(st.kp, st.vp, n, 8 * k)
+    keys, vals = col.result()
+    want = np.repeat(np.arange(len(pieces)), pieces)
+    assert np.array_equal(vals, want) and np.array_equal(keys.reshape(-1), np.repeat(want, kw))
+    for a in (keys, vals):
+        assert (a if a.base is None else a.base).nbytes == a.nbytes
