@@ -96,7 +96,7 @@ EXPORTS = [
     "gsparc_serve_create", "gsparc_serve_destroy", "gsparc_serve_upload", "gsparc_serve_release",
     "gsparc_serve_submit", "gsparc_serve_poll", "gsparc_serve_wait", "gsparc_serve_stats",
     "gsparc_serve_reset_stats", "gsparc_serve_pause", "gsparc_serve_inject_alloc_failure",
-    "gsparc_ctx_inject_alloc_failure", "gsparc_sptc_host", "gsparc_sptc_resident", "gsparc_tensor_download",
+    "gsparc_ctx_inject_alloc_failure", "gsparc_ctx_inject_scan_failure", "gsparc_sptc_host", "gsparc_sptc_resident", "gsparc_tensor_download",
     "gsparc_read_quantum", "gsparc_autotune", "gsparc_plan_create", "gsparc_plan_chunks", "gsparc_plan_chunk",
     "gsparc_plan_job_output", "gsparc_plan_refresh", "gsparc_plan_execute", "gsparc_plan_check",
     "gsparc_plan_destroy", "gsparc_tensor_set_values",
@@ -223,6 +223,7 @@ def lib():
     L.gsparc_serve_pause.argtypes = [P, I]
     L.gsparc_serve_inject_alloc_failure.argtypes = [P, U64]
     L.gsparc_ctx_inject_alloc_failure.argtypes = [P, U64]
+    L.gsparc_ctx_inject_scan_failure.argtypes = [P, I]
     for name in EXPORTS:
         getattr(L, name).restype = getattr(L, name).restype if name in (
             "gsparc_version", "gsparc_status_string", "gsparc_last_error") else (
@@ -442,6 +443,12 @@ class Context:
         """Host-side fault injection: the nth device allocation of this context
         from now (1 = the next) fails with GSPARC_ENOMEM, once; 0 disarms."""
         _check(lib().gsparc_ctx_inject_alloc_failure(self._h, nth), "ctx_inject_alloc_failure")
+
+    def inject_scan_failure(self, which: int):
+        """Host-side fault injection: the next contraction finds the error bit of
+        a prefix sum whose wait gave up (1: output offsets, 2: units of rows over
+        few columns, 3: those of its output chunks) and fails, once; 0 disarms."""
+        _check(lib().gsparc_ctx_inject_scan_failure(self._h, which), "ctx_inject_scan_failure")
 
     def set_tiles(self, light_row_max: int = 0, heavy_window_cap: int = 0):
         """Accumulation tiles of later contractions (0 = defaults): rows of up to

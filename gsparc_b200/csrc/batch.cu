@@ -39,6 +39,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kMaxGroupJobs = 65535;      // row_job is 16 bits
 constexpr uint64_t kMaxGroupNnz = (1ull << 31) - 1;
+constexpr char kLookBackGaveUp[] = "a prefix sum's or the radix sort's look-back gave up";
 
 inline int grid_for(uint64_t n) {
     uint64_t g = (n + kThreads - 1) / kThreads;
@@ -593,6 +594,15 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     DBuf<uint64_t> scan_vals(A, std::max({scan_value_words<1>(ny), col_bits ? scan_value_words<1>(col_words) : 0,
                                           scan_value_words<kMaxScanSums>(nx)}), s);
     auto scan_state = [&](uint32_t *flags) { return ScanState{flags, scan_vals.get(), plan_err}; };
+    // The scans after the first readback report to the context's error word,
+    // which is read again after the symbolic pass and at the end.
+    auto late_scan = [&](uint32_t *flags, int which) {
+        if (ctx->inject_scan == which) {
+            ctx->inject_scan = 0;
+            GS_CUDA(cudaMemsetAsync(ctx->d_flag, (int)kScanErr, 1, s));
+        }
+        return ScanState{flags, scan_vals.get(), ctx->d_flag};
+    };
     std::vector<uint8_t> h_tabs(tab_bytes);
     std::memcpy(h_tabs.data(), lx.data(), o_ly);
     std::memcpy(h_tabs.data() + o_ly, ly.data(), o_ly);
@@ -819,7 +829,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     std::memcpy(jerr.data(), head + sizeof(hc_cnt), 4 * (size_t)g);
     unsigned int herr = (unsigned int)hc_cnt[kCntErr];
     uint64_t ir = hc_cnt[kCntProducts];
-    GS_REQUIRE(!(herr & kScanErr), GSPARC_EINTERNAL, "a prefix sum's or the radix sort's look-back gave up");
+    GS_REQUIRE(!(herr & kScanErr), GSPARC_EINTERNAL, kLookBackGaveUp);
     const uint64_t bm_words_all = hc_cnt[kCntBmAll], bm_words_dense = hc_cnt[kCntBmDense];
     const uint64_t nrows = hc_cnt[kCntRows], nh = hc_cnt[kCntHeavy], nl = hc_cnt[kCntLight],
                    nu = hc_cnt[kCntUnits], nsr = hc_cnt[kCntStream];
@@ -938,7 +948,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         part.reset(A, std::max<uint64_t>(nparts, 1), s);
         GS_CUDA(cudaMemsetAsync(nbm.get(), 0, 4 * nbm_words, s));
         launch_narrow_units(Hs, (uint32_t)nh, row_class, row_prod, slice, unit_off, part_off,
-                            scan_state(flags_x + 4 * zf_x), s);
+                            late_scan(flags_x + 4 * zf_x, 2), s);
         aa.row_class = row_class;
         aa.unit_off = unit_off;
         aa.part_off = part_off;
@@ -1001,7 +1011,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
             launch_narrow(b, false, ctx->sm_count, s);
         }
     }
-    launch_row_offsets(row_nnz, nrows, row_off, scan_state(flags_x + 6 * zf_x), s);
+    launch_row_offsets(row_nnz, nrows, row_off, late_scan(flags_x + 6 * zf_x, 1), s);
     const UnitLists ul{L, nl, H, nh, SR, nsr};
     k_after_counts<<<grid_for(std::max<uint64_t>(nl + nh + nsr, (uint64_t)g + 1)), kThreads, 0, s>>>(
         ul, row_off, row_job, nrows, xprefix, d_xoffs, g, ctx->d_flag, d_jo);
@@ -1017,6 +1027,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     herr = (unsigned int)jo[g + 1].out_off;
     bst.bytes_d2h += sizeof(JobOut) * (g + 1) + 64 + 4 * g + 8;
     GS_REQUIRE(!(herr & 2u), GSPARC_EINTERNAL, "light unit over capacity");
+    GS_REQUIRE(!(herr & kScanErr), GSPARC_EINTERNAL, kLookBackGaveUp);
     const uint64_t ntot = jo[g].out_off;
     bst.nnz += ntot;
     mark(4);
@@ -1124,7 +1135,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     bst.chunks += chunks.size();
     if (nnarrow && Hchunk != Hs)  // the chunks' own order
         launch_narrow_units(Hchunk, (uint32_t)nh, row_class, row_prod, slice, unit_off, part_off,
-                            scan_state(flags_x + 5 * zf_x), s);
+                            late_scan(flags_x + 5 * zf_x, 3), s);
 
     if (keep) {
         // a plan keeps what the numeric pass needs and stops here
@@ -1197,7 +1208,10 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         keep->aa.err = keep->flags.get();
         keep->aa.work_counter = keep->flags.get() + 1;
         keep->aa.row_nnz = nullptr;  // the symbolic counts are not kept
+        unsigned int e = 0;
+        d2h(&e, ctx->d_flag, 1, s);
         GS_CUDA(cudaStreamSynchronize(s));
+        GS_REQUIRE(!(e & kScanErr), GSPARC_EINTERNAL, kLookBackGaveUp);
         tm.lin += ms(0, 1);
         tm.sort += ms(1, 2);
         tm.match += ms(2, 3);
@@ -1348,7 +1362,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
             unsigned int e = 0;
             d2h(&e, ctx->d_flag, 1, s2);
             GS_CUDA(cudaStreamSynchronize(s2));
-            GS_REQUIRE(!(e & 6u), GSPARC_EINTERNAL, "numeric pass failed a device-side check");
+            GS_REQUIRE(!(e & (6u | kScanErr)), GSPARC_EINTERNAL, "numeric pass failed a device-side check");
         }
         if (done_fn)
             for (; next_done < g && job_first[next_done + 1] <= c1; ++next_done) {
@@ -1394,6 +1408,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     GS_CUDA(cudaStreamSynchronize(s));
     bst.heavy_windows += hflags[2];
     GS_REQUIRE(!(hflags[0] & 2u), GSPARC_EINTERNAL, "light unit over capacity");
+    GS_REQUIRE(!(hflags[0] & kScanErr), GSPARC_EINTERNAL, kLookBackGaveUp);
     GS_REQUIRE(!(hflags[0] & 4u), GSPARC_EINTERNAL, "numeric pass wrote past its chunk (symbolic count mismatch)");
     tm.lin += ms(0, 1);
     tm.sort += ms(1, 2);

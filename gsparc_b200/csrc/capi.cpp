@@ -131,6 +131,14 @@ gsparc_status gsparc_ctx_inject_alloc_failure(gsparc_ctx *ctx, uint64_t nth) {
     });
 }
 
+gsparc_status gsparc_ctx_inject_scan_failure(gsparc_ctx *ctx, int which) {
+    return guard([&] {
+        GS_REQUIRE(ctx, GSPARC_EINVAL, "null context");
+        GS_REQUIRE(which >= 0 && which <= 3, GSPARC_EINVAL, "which must be 0..3");
+        ctx->inject_scan = which;
+    });
+}
+
 gsparc_status gsparc_ctx_set_tiles(gsparc_ctx *ctx, uint64_t light_row_max, uint32_t heavy_window_cap) {
     return guard([&] {
         GS_REQUIRE(ctx, GSPARC_EINVAL, "null context");

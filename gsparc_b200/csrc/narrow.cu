@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(NT) k_narrow(AccArgs a) {
     const uint32_t le = 0xffffffffu >> (31 - lane);
     float2 *my = acc + warp * ncp;
     uint8_t *tag = tags + warp * ncp;
+    if (*a.err & kScanErr) return;  // the units were not written
     const uint32_t ubase = a.unit_off[0], nunits = a.unit_off[a.nunits] - ubase;
     if (NUMERIC)
         for (uint32_t c = tid; c < NW * ncp; c += NT) acc[c] = make_float2(0.f, 0.f);
@@ -311,6 +312,7 @@ __global__ void __launch_bounds__(NT) k_narrow(AccArgs a) {
 
 // Rows of several units: their partial pairs in unit order.  A CTA per row.
 __global__ void __launch_bounds__(NT) k_narrow_sum(AccArgs a) {
+    if (*a.err & kScanErr) return;
     for (uint32_t at = blockIdx.x; at < a.nunits; at += gridDim.x) {
         const uint32_t nu = a.unit_off[at + 1] - a.unit_off[at];
         if (nu < 2) continue;

@@ -187,6 +187,11 @@ gsparc_status gsparc_ctx_set_verify(gsparc_ctx *ctx, uint64_t max_products);
  * nth device allocation of this context from now (1 = the next) fails with
  * GSPARC_ENOMEM, once; 0 disarms.  The device is not involved. */
 gsparc_status gsparc_ctx_inject_alloc_failure(gsparc_ctx *ctx, uint64_t nth);
+/* The same for a prefix sum whose wait gives up: the next contraction of this
+ * context finds the error bit such a wait leaves (1: with the output offsets,
+ * 2: with the units of rows over few columns, 3: with those of its output
+ * chunks) and fails with GSPARC_EINTERNAL, once; 0 disarms.  No wait runs out. */
+gsparc_status gsparc_ctx_inject_scan_failure(gsparc_ctx *ctx, int which);
 /* Bytes currently allocated by the context and its high-water mark. */
 gsparc_status gsparc_ctx_memory(gsparc_ctx *ctx, uint64_t *in_use, uint64_t *peak,
                                 uint64_t *budget);
