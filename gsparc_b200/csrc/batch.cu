@@ -25,6 +25,7 @@
 #include <cstring>
 #include <numeric>
 
+#include "chunkkey.h"
 #include "engine.h"
 #include "kernels.cuh"
 #include "rows.h"
@@ -361,12 +362,10 @@ __global__ void k_chunk_bounds(const uint32_t *__restrict__ urow, const uint64_t
     }
 }
 
-// Sort key grouping heavy rows by chunk, inside a chunk the windowed kernel's
-// rows before the narrow rows, largest first.
+// Sort keys grouping heavy rows by chunk (chunkkey.h).
 __global__ void k_heavy_chunk_keys(const uint32_t *__restrict__ Hs, uint64_t nh,
                                    const uint64_t *__restrict__ row_prod, const uint8_t *__restrict__ row_class,
                                    const uint64_t *__restrict__ info, uint64_t K, uint64_t *__restrict__ keys) {
-    constexpr uint64_t kProdMask = (1ull << 44) - 1;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nh; k += stride) {
         const uint32_t r = Hs[k];
@@ -378,9 +377,7 @@ __global__ void k_heavy_chunk_keys(const uint32_t *__restrict__ Hs, uint64_t nh,
             else
                 hi = mid;
         }
-        const uint64_t p = row_prod[r];
-        const uint64_t narrow = row_class && row_class[r] == kRowNarrow;
-        keys[k] = (lo << 45) | (narrow << 44) | (kProdMask - (p < kProdMask ? p : kProdMask));
+        keys[k] = heavy_chunk_key(lo, row_class && row_class[r] == kRowNarrow, row_prod[r]);
     }
 }
 
@@ -1116,7 +1113,8 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
             k_heavy_chunk_keys<<<grid_for(nh), kThreads, 0, s>>>(Hs, nh, row_prod, aa.row_class, cinfo, K, hk0);
             count_launch();
             GS_CUDA(cudaGetLastError());
-            const int bits = 45 + ceil_log2(K);
+            const int bits = kChunkProdBits + 1 + ceil_log2(K);
+            GS_REQUIRE(bits <= 64, GSPARC_EINTERNAL, "too many output chunks");
             size_t tmp = 0;
             GS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, hk0.get(), hk1.get(), Hs, Hc.get(), (int)nh, 0,
                                                     bits, s));

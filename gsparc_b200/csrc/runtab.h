@@ -5,11 +5,7 @@
 
 #include <cstdint>
 
-#ifdef __CUDACC__
-#define GS_HD __host__ __device__ __forceinline__
-#else
-#define GS_HD inline
-#endif
+#include "hd.h"
 
 namespace gs {
 
