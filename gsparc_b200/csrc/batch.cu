@@ -756,6 +756,8 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
                                                     ctab, pos, cnt, rflag);
         count_launch();
         GS_CUDA(cudaGetLastError());
+        run_key.release();
+        run_start.release();
         RowArrays ra{};
         ra.xprefix = xprefix;
         ra.mpre = mpre;
@@ -786,6 +788,8 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
             ra.row_mx = row_mx;
         }
         launch_x_rows(xkeys, nx, kbx, d_bp, cnt, rflag, ra, cnts, scan_state(flags_x), s);
+        xk0.release();
+        xk1.release();
         if (any_wide)
             launch_wide_tables(reinterpret_cast<const WideTab *>(tabs.get() + o_wt), g, std::max(nx, ny), row_job, row_xf,
                                cols, d_acc, cnts, plan_err, s);
@@ -853,16 +857,59 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     const uint64_t nnarrow = fits(4 * nbm_words + 8 * nparts, 16) ? hc_cnt[kCntNarrow] : 0;
     const uint8_t *narrow_class = nnarrow ? row_class.get() : nullptr;
 
-    // y_f of every Y entry for the heavy rows, where it fits 32 bits and the memory allows
+    // What no later pass of this group reads goes back before anything else is
+    // taken.  The planning's arrays are sized for a row an X nonzero, so that the
+    // output and the heavy rows' cursors have more need of them: with all of them
+    // held, 6e5 rows beside a row of 1e6 outputs needed 196 MB, now 162.
+    const auto free_light = [&] {
+        ustart.release();
+        lk0.release();
+        lrun.release();
+        lrow.release();
+        lpre.release();
+        loff.release();
+    };
+    if (!nl) {
+        free_light();
+        L.release();
+    }
+    if (!nsr) {
+        SR.release();
+        sprefix.release();
+    }
+    if (!nh) {
+        H.release();
+        row_prod.release();
+        row_rb.release();
+        bm_w_all.release();
+        bm_w_dense.release();
+        bm_off_all.release();
+        bm_off_dense.release();
+    }
+    if (!nnarrow) {
+        mpre.release();
+        mrun.release();
+        row_class.release();
+    }
+
+    // y_f of every Y entry for the heavy rows, where it fits 32 bits, the memory
+    // allows, and rows past the light ones have a product for every entry
     DBuf<uint32_t> ycol;
     {
         int most = 0;
         for (Job *q : G)
             most = std::max(most, q->wide && q->key_words == 1 ? q->wide->nfbits_y : q->LY.nfbits);
-        if (nh > nnarrow && most <= 32 && fits(4 * ny, 16)) {
+        if (nh > nnarrow && most <= 32 && ir - hc_cnt[kCntLightProd] >= ny && fits(4 * ny, 16)) {
             ycol.reset(A, ny, s);
             launch_y_cols32(ykeys, ny, kby, d_acc, cols, rank, ycol, plan_err, s);
         }
+    }
+
+    if (!nsr) {  // single-run rows alone take y_f from the sorted keys
+        yk0.release();
+        yk1.release();
+        if (keep) keep->ykeys.release();
+        ykeys = nullptr;
     }
 
     // heavy rows largest first (H itself stays in row order for chunk planning)
@@ -884,7 +931,11 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     }
 
     // ---- symbolic pass ----
-    DBuf<uint32_t> cursor(A, nxb, s), pend(A, nxb, s);
+    DBuf<uint32_t> cursor, pend;  // of the windowed kernel
+    if (nh > nnarrow) {
+        cursor.reset(A, nxb, s);
+        pend.reset(A, nxb, s);
+    }
     DBuf<uint64_t> row_off(A, nrows + 1, s);
     AccArgs aa{};
     aa.row_job = row_job;
@@ -1009,6 +1060,10 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         }
     }
     launch_row_offsets(row_nnz, nrows, row_off, late_scan(flags_x + 6 * zf_x, 1), s);
+    row_nnz.release();
+    aa.row_nnz = nullptr;
+    if (light_once) free_light();
+    if (!bm_off) row_rb.release();
     const UnitLists ul{L, nl, H, nh, SR, nsr};
     k_after_counts<<<grid_for(std::max<uint64_t>(nl + nh + nsr, (uint64_t)g + 1)), kThreads, 0, s>>>(
         ul, row_off, row_job, nrows, xprefix, d_xoffs, g, ctx->d_flag, d_jo);
@@ -1134,9 +1189,48 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     if (nnarrow && Hchunk != Hs)  // the chunks' own order
         launch_narrow_units(Hchunk, (uint32_t)nh, row_class, row_prod, slice, unit_off, part_off,
                             late_scan(flags_x + 5 * zf_x, 3), s);
+    row_prod.release();
 
     if (keep) {
-        // a plan keeps what the numeric pass needs and stops here
+        // a plan keeps what the numeric pass needs, in arrays of the sizes that
+        // turned out (a copy each, where the memory has room for it), and stops here
+        const auto fit = [&](auto &b, uint64_t n, auto &at) {
+            using T = std::remove_reference_t<decltype(*b.get())>;
+            n = std::max<uint64_t>(n, 1);
+            if (b.size() <= n || sizeof(T) * n + 256 > A.available()) return;
+            std::remove_reference_t<decltype(b)> c(A, n, s);
+            GS_CUDA(cudaMemcpyAsync(c.get(), b.get(), sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
+            b = std::move(c);
+            at = b.get();
+        };
+        if (Hc.get()) H2.release();  // the list that heavy_list() takes
+        if (Hc.get() || H2.get()) H.release();
+        const uint32_t *list = nullptr;  // the lists' addresses are taken when a chunk is launched
+        fit(L, nl, list);
+        fit(H, nh, list);
+        fit(SR, nsr, list);
+        const uint64_t *pre = nullptr;
+        fit(sprefix, nsr + 1, pre);
+        fit(ustart, nu + 1, aa.ustart);
+        fit(lk0, nl + 1, aa.lk0);
+        fit(lpre, nl + 1, aa.lpre);
+        fit(lrun, hc_cnt[kCntLightRuns], aa.lrun);
+        fit(lrow, hc_cnt[kCntLightRuns], aa.lrow);
+        fit(loff, hc_cnt[kCntLightRuns], aa.loff);
+        fit(row_start, nrows + 1, aa.row_start);
+        fit(row_xf, nrows, aa.row_xf);
+        fit(row_job, nrows, aa.row_job);
+        fit(row_xi, nrows, aa.row_xi);
+        if (aa.col_is_key && !nl && !nnarrow && !any_wide)
+            cols.release();  // no row looks a column up
+        else
+            fit(cols, hc_cnt[kCntCols], aa.cols);
+        if (nnarrow) fit(row_class, nrows, aa.row_class);
+        if (bm_off) {
+            fit(row_rb, nrows, aa.row_rb);
+            fit(*bm_off, nrows, aa.row_bmoff);
+            fit(bm_off == &bm_off_all ? bm_w_all : bm_w_dense, nrows, aa.row_bmw);
+        }
         keep->g = g;
         keep->nx = nx;
         keep->ny = ny;
@@ -1205,7 +1299,6 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         keep->aa = aa;  // the moved buffers keep their device addresses
         keep->aa.err = keep->flags.get();
         keep->aa.work_counter = keep->flags.get() + 1;
-        keep->aa.row_nnz = nullptr;  // the symbolic counts are not kept
         unsigned int e = 0;
         d2h(&e, ctx->d_flag, 1, s);
         GS_CUDA(cudaStreamSynchronize(s));

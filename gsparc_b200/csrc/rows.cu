@@ -420,6 +420,7 @@ __global__ void __launch_bounds__(kScanThreads)
         cnts[kCntLight] = (uint32_t)sh.through[1];
         cnts[kCntNarrow] = sh.through[1] >> 32;
         cnts[kCntLightProd] = sh.through[2];
+        cnts[kCntLightRuns] = (uint32_t)sh.through[4];
         r.lpre[(uint32_t)sh.through[1]] = sh.through[2];
         r.lk0[(uint32_t)sh.through[1]] = (uint32_t)sh.through[4];
         r.sprefix[sh.through[0] >> 32] = sh.through[3];

@@ -33,7 +33,8 @@ enum {
     kCntNarrowCols = 15, // most columns of a job with narrow rows
     kCntProducts = 16,
     kCntErr = 17,        // error bits of the planning kernels and the radix sort (low word)
-    kCnts = 18
+    kCntLightRuns = 18,  // runs of the light rows
+    kCnts = 19
 };
 
 constexpr uint8_t kRowNone = 0, kRowLight = 1, kRowStream = 2, kRowHeavy = 3, kRowNarrow = 4;  // narrow: heavy, over few columns
