@@ -512,6 +512,14 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         GS_CUDA(cudaEventElapsedTime(&t, ev[a], ev[b]));
         return (double)t;
     };
+    // The operands' stages run side by side: one ends when both operands are
+    // through it (events 1, 2: Y, 10, 9: X).
+    auto operand_times = [&] {
+        const double lin = std::max(ms(0, 1), ms(0, 10)), sorted = std::max(ms(0, 2), ms(0, 9));
+        tm.lin += lin;
+        tm.sort += sorted - lin;
+        tm.match += std::max(ms(0, 3) - sorted, 0.0);
+    };
     mark(0);
 
     // ---- job tables ----
@@ -645,6 +653,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         count_launch();
         GS_CUDA(cudaGetLastError());
     }
+    GS_CUDA(cudaEventRecord(ev[10], sx));
     // gsparc_ctx_set_sort; a failed look-back sets bit 8 of the error word
     if (ctx->sort_impl)
         own_sort_pairs(A, nx, xk0, xk1, xv0, xv1, kbx + jb, &wx, plan_err, sx, xbegin);
@@ -1303,9 +1312,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         d2h(&e, ctx->d_flag, 1, s);
         GS_CUDA(cudaStreamSynchronize(s));
         GS_REQUIRE(!(e & kScanErr), GSPARC_EINTERNAL, kLookBackGaveUp);
-        tm.lin += ms(0, 1);
-        tm.sort += ms(1, 2);
-        tm.match += ms(2, 3);
+        operand_times();
         tm.plan += ms(3, 4);
         tm.total += ms(0, 4);
         return;
@@ -1501,9 +1508,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     GS_REQUIRE(!(hflags[0] & 2u), GSPARC_EINTERNAL, "light unit over capacity");
     GS_REQUIRE(!(hflags[0] & kScanErr), GSPARC_EINTERNAL, kLookBackGaveUp);
     GS_REQUIRE(!(hflags[0] & 4u), GSPARC_EINTERNAL, "numeric pass wrote past its chunk (symbolic count mismatch)");
-    tm.lin += ms(0, 1);
-    tm.sort += ms(1, 2);
-    tm.match += ms(2, 3);
+    operand_times();
     tm.plan += ms(3, 4);
     tm.contract += ms(4, 5);
     tm.total += ms(0, 5);

@@ -105,9 +105,11 @@ typedef struct {
     uint64_t chunks;          /* output chunks streamed                       */
     int nbits_x, nbits_y, ncbits, nfbits_x, nfbits_y;
     int accumulator;          /* accumulator actually used (GSPARC_ACCUM_*)   */
+    /* X and Y are linearised and sorted side by side: a stage ends when both
+     * operands are through it (Y's tables may be made while X is still sorted) */
     double t_linearize_ms;    /* SLITOM construction (linearise)              */
     double t_sort_ms;         /* SLITOM sort                                  */
-    double t_match_ms;        /* index match + row table                      */
+    double t_match_ms;        /* Y's tables, index match + row table          */
     double t_plan_ms;         /* symbolic pass + chunk planning               */
     double t_contract_ms;     /* numeric accumulation                         */
     double t_output_ms;       /* output delivery (copies, callbacks)          */
