@@ -556,10 +556,22 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
                                          (A.available() - std::min(A.available(), plan_need)) / 4);
     const bool col_bits = col_words * 8 <= table_most;
     // The run lookup table (8 B per 32 contract keys) under the same bounds.
-    // With it the match does not care for the order of a row's nonzeros, so X
-    // is sorted by its free bits alone.  1e7 x 1e7 nonzeros over 2^24 contract
-    // keys: X's radix passes 4 -> 1 (122 us each), match 241 -> 101 us.
+    // 1e7 x 1e7 nonzeros over 2^24 contract keys: match 241 -> 101 us.
     const bool con_tab = con_words * 8 <= table_most;
+    // With the table the match does not care for the order of a row's nonzeros, so
+    // X may be sorted by its free bits alone (at the size above 4 -> 1 radix passes
+    // of 122 us).  Light rows add in the order of their contract keys whatever the
+    // input's order and the jobs beside them, so theirs are put in it afterwards
+    // (launch_light_order), which pays where X has at least twice as many nonzeros
+    // for every free index as a light row may have products: few rows are light
+    // then, and all of them together have at most nx / 2 runs to sort.
+    bool by_free = con_tab;
+    uint64_t free_rows = 0;  // free indices of the jobs that may have light rows
+    for (Job *q : G) {
+        const int fb = q->LX.nfbits;
+        by_free &= !q->light_max || (fb < 32 && q->tx->nnz >= (2 * q->light_max) << fb);
+        if (q->light_max && fb < 32) free_rows += 1ull << fb;
+    }
     // relabeled jobs with 64-bit output keys
     bool any_wide = false;
     for (Job *q : G) any_wide |= q->wide && q->key_words == 1;
@@ -646,7 +658,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     GS_CUDA(cudaEventRecord(ev[8], s));
     GS_CUDA(cudaStreamWaitEvent(sx, ev[8], 0));
     join.sx = sx;
-    const int xbegin = con_tab ? min_ncb : 0;
+    const int xbegin = by_free ? min_ncb : 0;
     int wx = 0, wy = 0;
     if (nx) {
         k_blin<<<grid_for(nx), kThreads, 0, sx>>>(d_lx, d_xoffs, g, nx, kbx, xk0, xv0, d_jerr, keep != nullptr);
@@ -814,6 +826,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         mark(3);
         launch_light_units(nx, light_bin, ra, cnts, scan_state(flags_x + 2 * zf_x), s);
         launch_matched_runs(nx, pos, cnt, rank, ra, cnts, plan_err, s);
+        if (by_free) launch_light_order(free_rows, pos, cnt, ra, cnts, plan_err, ctx->sm_count, s);
         if (keep_bm)
             launch_heavy_bitmaps(nx, ra, bm_w_all, bm_w_dense, bm_off_all, bm_off_dense, cnts,
                                  scan_state(flags_x + 3 * zf_x), s);

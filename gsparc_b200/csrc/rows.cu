@@ -509,6 +509,62 @@ __global__ void k_matched_runs(const uint32_t *__restrict__ pos, const uint32_t 
     }
 }
 
+// Where X is sorted by its free bits alone, a CTA a light row: its runs in the
+// order of their contract keys (the order of their first Y entries), equal keys
+// in input order, as the sort by all bits leaves them.  So a light row's sums
+// depend neither on the order of the input nor on the jobs beside it.  Rows are
+// long there (batch.cu, by_free), so few are light: with none, 3 us.
+constexpr int kOrderRuns = 2048;  // a light row has no more products
+static_assert(kOrderRuns >= kLightCap / 2, "the largest light_row_max");
+__global__ void __launch_bounds__(kThreads)
+    k_light_order(const uint32_t *__restrict__ pos, const uint32_t *__restrict__ cnt, RowArrays r,
+                  const uint64_t *__restrict__ cnts, const unsigned int *__restrict__ err) {
+    constexpr int kPer = kOrderRuns / kThreads;
+    __shared__ uint64_t key[kOrderRuns];  // first Y entry, X nonzero
+    __shared__ uint32_t s_tmp[33];
+    if (*err & kScanErr) return;
+    const uint32_t n = (uint32_t)cnts[kCntLight], tid = threadIdx.x;
+    for (uint32_t l = blockIdx.x; l < n; l += gridDim.x) {
+        const uint32_t a = r.lk0[l], m = min(r.lk0[l + 1] - a, (uint32_t)kOrderRuns);
+        uint32_t padded = 1;
+        while (padded < m) padded <<= 1;
+        __syncthreads();  // the row before this one has left `key`
+        for (uint32_t t = tid; t < padded; t += kThreads) {
+            const uint32_t i = t < m ? r.lrun[a + t] : 0u;
+            key[t] = t < m ? (uint64_t)pos[i] << 32 | i : ~0ull;
+        }
+        __syncthreads();
+        for (uint32_t k = 2; k <= padded; k <<= 1)
+            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+                for (uint32_t t = tid; t < padded / 2; t += kThreads) {
+                    const uint32_t lo = ((t & ~(j - 1)) << 1) | (t & (j - 1)), hi = lo | j;
+                    const uint64_t x = key[lo], y = key[hi];
+                    if ((x > y) == ((lo & k) == 0)) {
+                        key[lo] = y;
+                        key[hi] = x;
+                    }
+                }
+                __syncthreads();
+            }
+        uint32_t c[kPer], sum = 0, all;
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const uint32_t t = tid * kPer + q;
+            c[q] = sum;
+            if (t < m) sum += cnt[(uint32_t)key[t]];
+        }
+        const uint32_t before = block_excl_scan_u32<kThreads>(sum, s_tmp, &all);
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            const uint32_t t = tid * kPer + q;
+            if (t < m) {
+                r.lrun[a + t] = (uint32_t)key[t];
+                r.loff[a + t] = r.lpre[l] + before + c[q];
+            }
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kScanThreads)
     k_heavy_words(RowArrays r, uint32_t *__restrict__ w_all, uint32_t *__restrict__ w_dense, uint64_t *__restrict__ off_all,
                   uint64_t *__restrict__ off_dense, uint64_t *__restrict__ cnts, ScanState st) {
@@ -647,6 +703,13 @@ void launch_matched_runs(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, 
                          const RowArrays &r, const uint64_t *cnts, const unsigned int *err, cudaStream_t s) {
     if (nx == 0) return;
     k_matched_runs<<<grid_for(nx), kThreads, 0, s>>>(pos, cnt, yrank, r, cnts, err);
+    launched();
+}
+
+void launch_light_order(uint64_t rows, const uint32_t *pos, const uint32_t *cnt, const RowArrays &r,
+                        const uint64_t *cnts, const unsigned int *err, int sm_count, cudaStream_t s) {
+    if (rows == 0) return;
+    k_light_order<<<(unsigned)std::min<uint64_t>(rows, 8ull * sm_count), kThreads, 0, s>>>(pos, cnt, r, cnts, err);
     launched();
 }
 

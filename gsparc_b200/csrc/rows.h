@@ -105,6 +105,11 @@ void launch_light_units(uint64_t nx, uint64_t bin, const RowArrays &r, uint64_t 
 // span of every heavy row.
 void launch_matched_runs(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, const uint32_t *yrank,
                          const RowArrays &r, const uint64_t *cnts, const unsigned int *err, cudaStream_t s);
+// Where X is sorted by its free bits alone: the light rows' runs (lrun, loff) in
+// the order of their contract keys, equal ones in input order.  `rows`: the most
+// light rows there can be.
+void launch_light_order(uint64_t rows, const uint32_t *pos, const uint32_t *cnt, const RowArrays &r,
+                        const uint64_t *cnts, const unsigned int *err, int sm_count, cudaStream_t s);
 // Kept bitmaps: of every heavy row the words with all / only dense
 // rows kept (w_*, by row), their word offsets (off_*, by row) and totals.
 void launch_heavy_bitmaps(uint64_t nx, const RowArrays &r, uint32_t *w_all, uint32_t *w_dense,
