@@ -307,6 +307,9 @@ def plan_shards(row_prod: np.ndarray, nshards: int) -> np.ndarray:
 
 # ------------------------------------------------------------------ host staging
 STAGING_NNZ = 1 << 18  # output nonzeros of a kept staging buffer (3 MiB page-locked)
+# Spare nonzeros (12 B each, mostly pages that were never touched) that a result
+# may keep: cutting 8 MiB arrays to 4 cost 1 ms of page faults in the next calls.
+SPARE_NNZ = 1 << 21
 
 
 class _Staging:
@@ -386,7 +389,7 @@ class _CallerStaging:
 class _Collect:
     """Gathers the pieces a HOST sink delivers (in order, through `st`) into
     result arrays: exactly sized when one piece is all, grown by doubling and
-    cut to size at the end otherwise."""
+    cut to size at the end (SPARE_NNZ) otherwise."""
 
     def __init__(self, st: _Staging, kw: int = 1):
         self.st, self.kw, self.n = st, kw, 0
@@ -414,6 +417,9 @@ class _Collect:
     def result(self):
         if self.vals is None:
             return np.zeros((0, 2) if self.kw == 2 else 0, np.uint64), np.zeros(0, np.float32)
+        if self.vals.shape[0] - self.n <= SPARE_NNZ:
+            keys, vals = self.keys[: self.kw * self.n], self.vals[: self.n]
+            return (keys.reshape(-1, 2) if self.kw == 2 else keys), vals
         # the grown arrays' spare end goes back to the system (nothing else refers to them)
         self.keys.resize(self.kw * self.n, refcheck=False)
         self.vals.resize(self.n, refcheck=False)

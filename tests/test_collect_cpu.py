@@ -118,7 +118,8 @@ def test_dropped_staging_is_unregistered(monkeypatch):
 
 @pytest.mark.parametrize("kw", [1, 2])
 @pytest.mark.parametrize("pieces", [[8], [8, 1], [8] * 5 + [3], [8] * 300 + [1]])
-def test_results_hold_no_spare_memory(kw, pieces):
+def test_results_hold_no_spare_memory(monkeypatch, kw, pieces):
+    monkeypatch.setattr(api, "SPARE_NNZ", 0)
     st = _Plain(kw * 8)
     col = api._Collect(st, kw)
     for k, n in enumerate(pieces):
