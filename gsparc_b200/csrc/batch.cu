@@ -879,41 +879,6 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     const uint64_t nnarrow = fits(4 * nbm_words + 8 * nparts, 16) ? hc_cnt[kCntNarrow] : 0;
     const uint8_t *narrow_class = nnarrow ? row_class.get() : nullptr;
 
-    // What no later pass of this group reads goes back before anything else is
-    // taken.  The planning's arrays are sized for a row an X nonzero, so that the
-    // output and the heavy rows' cursors have more need of them: with all of them
-    // held, 6e5 rows beside a row of 1e6 outputs needed 196 MB, now 162.
-    const auto free_light = [&] {
-        ustart.release();
-        lk0.release();
-        lrun.release();
-        lrow.release();
-        lpre.release();
-        loff.release();
-    };
-    if (!nl) {
-        free_light();
-        L.release();
-    }
-    if (!nsr) {
-        SR.release();
-        sprefix.release();
-    }
-    if (!nh) {
-        H.release();
-        row_prod.release();
-        row_rb.release();
-        bm_w_all.release();
-        bm_w_dense.release();
-        bm_off_all.release();
-        bm_off_dense.release();
-    }
-    if (!nnarrow) {
-        mpre.release();
-        mrun.release();
-        row_class.release();
-    }
-
     // y_f of every Y entry for the heavy rows, where it fits 32 bits, the memory
     // allows, and rows past the light ones have a product for every entry
     DBuf<uint32_t> ycol;
@@ -925,13 +890,6 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
             ycol.reset(A, ny, s);
             launch_y_cols32(ykeys, ny, kby, d_acc, cols, rank, ycol, plan_err, s);
         }
-    }
-
-    if (!nsr) {  // single-run rows alone take y_f from the sorted keys
-        yk0.release();
-        yk1.release();
-        if (keep) keep->ykeys.release();
-        ykeys = nullptr;
     }
 
     // heavy rows largest first (H itself stays in row order for chunk planning)
@@ -1082,15 +1040,42 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         }
     }
     launch_row_offsets(row_nnz, nrows, row_off, late_scan(flags_x + 6 * zf_x, 1), s);
-    row_nnz.release();
-    aa.row_nnz = nullptr;
-    if (light_once) free_light();
-    if (!bm_off) row_rb.release();
     const UnitLists ul{L, nl, H, nh, SR, nsr};
     k_after_counts<<<grid_for(std::max<uint64_t>(nl + nh + nsr, (uint64_t)g + 1)), kThreads, 0, s>>>(
         ul, row_off, row_job, nrows, xprefix, d_xoffs, g, ctx->d_flag, d_jo);
     count_launch();
     GS_CUDA(cudaGetLastError());
+    // What no later pass of this group reads goes back before the output is taken,
+    // while the symbolic pass runs (between the readback and its launch the same
+    // cost 4 us a call).  The planning's arrays are sized for a row an X nonzero, so
+    // the output has more need of them: with all of them held, 6e5 rows beside a row
+    // of 1e6 outputs needed 196 MB, now 162.
+    row_nnz.release();
+    aa.row_nnz = nullptr;
+    if (!nl || light_once) {
+        ustart.release();
+        lk0.release();
+        lrun.release();
+        lrow.release();
+        lpre.release();
+        loff.release();
+    }
+    if (!nsr) {
+        SR.release();
+        sprefix.release();
+        // single-run rows alone take y_f from the sorted keys
+        yk0.release();
+        yk1.release();
+        if (keep) keep->ykeys.release();
+        aa.ykeys = nullptr;
+    }
+    if (!nh) row_prod.release();
+    if (!bm_off) row_rb.release();
+    if (!nnarrow) {
+        mpre.release();
+        mrun.release();
+        row_class.release();
+    }
     std::vector<JobOut> jo(g + 2);
     const size_t jo_bytes = sizeof(JobOut) * (size_t)(g + 2);
     void *jo_at = ctx->h_pin && jo_bytes <= gsparc_ctx::kPinBytes ? ctx->h_pin : jo.data();
