@@ -293,8 +293,8 @@ __global__ void __launch_bounds__(LightShape<C>::T) k_light(AccArgs a) {
                     v[q] = 0.f;
                     if (heads >> q & 1u) {
                         at = q;
-                        sum = pr[q];
-                        c = pe[q];
+                        sum = 0.f + pr[q];  // as from an empty accumulator: a product that
+                        c = 0.f + pe[q];    // underflows to -0 alone gives +0 on every path but the copied rows'
                     } else {
                         float ns, err;
                         two_sum(sum, pr[q], ns, err);
