@@ -507,18 +507,22 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
 
     cudaEvent_t *ev = ctx->ev;
     auto mark = [&](int i) { GS_CUDA(cudaEventRecord(ev[i], s)); };
-    auto ms = [&](int a, int b) {
+    auto at = [&](int i) {
         float t = 0.f;
-        GS_CUDA(cudaEventElapsedTime(&t, ev[a], ev[b]));
+        GS_CUDA(cudaEventElapsedTime(&t, ev[0], ev[i]));
         return (double)t;
     };
-    // The operands' stages run side by side: one ends when both operands are
-    // through it (events 1, 2: Y, 10, 9: X).
-    auto operand_times = [&] {
-        const double lin = std::max(ms(0, 1), ms(0, 10)), sorted = std::max(ms(0, 2), ms(0, 9));
+    // The stages up to the symbolic pass; returns where they end.  The operands'
+    // run side by side: one ends when both operands are through it (events 1, 2:
+    // Y, 10, 9: X).
+    auto planning_times = [&] {
+        const double lin = std::max(at(1), at(10)), sorted = std::max(at(2), at(9)), match = std::max(at(3), sorted);
+        const double end = at(4);
         tm.lin += lin;
         tm.sort += sorted - lin;
-        tm.match += std::max(ms(0, 3) - sorted, 0.0);
+        tm.match += match - sorted;
+        tm.plan += end - match;
+        return end;
     };
     mark(0);
 
@@ -1310,9 +1314,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         d2h(&e, ctx->d_flag, 1, s);
         GS_CUDA(cudaStreamSynchronize(s));
         GS_REQUIRE(!(e & kScanErr), GSPARC_EINTERNAL, kLookBackGaveUp);
-        operand_times();
-        tm.plan += ms(3, 4);
-        tm.total += ms(0, 4);
+        tm.total += planning_times();
         return;
     }
 
@@ -1506,10 +1508,9 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     GS_REQUIRE(!(hflags[0] & 2u), GSPARC_EINTERNAL, "light unit over capacity");
     GS_REQUIRE(!(hflags[0] & kScanErr), GSPARC_EINTERNAL, kLookBackGaveUp);
     GS_REQUIRE(!(hflags[0] & 4u), GSPARC_EINTERNAL, "numeric pass wrote past its chunk (symbolic count mismatch)");
-    operand_times();
-    tm.plan += ms(3, 4);
-    tm.contract += ms(4, 5);
-    tm.total += ms(0, 5);
+    const double planned = planning_times(), end = at(5);
+    tm.contract += end - planned;
+    tm.total += end;
     tm.out += t_out;
     // numeric kernel time: first chunk's start to the last chunk's end (chunks
     // on the two streams overlap)
