@@ -40,6 +40,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kMaxGroupJobs = 65535;      // row_job is 16 bits
 constexpr uint64_t kMaxGroupNnz = (1ull << 31) - 1;
+constexpr uint64_t kFreeSortNnz = 1ull << 12;
 constexpr char kLookBackGaveUp[] = "a prefix sum's or the radix sort's look-back gave up";
 
 inline int grid_for(uint64_t n) {
@@ -562,19 +563,23 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
     // The run lookup table (8 B per 32 contract keys) under the same bounds.
     // 1e7 x 1e7 nonzeros over 2^24 contract keys: match 241 -> 101 us.
     const bool con_tab = con_words * 8 <= table_most;
-    // With the table the match does not care for the order of a row's nonzeros, so
-    // X may be sorted by its free bits alone (at the size above 4 -> 1 radix passes
-    // of 122 us).  Light rows add in the order of their contract keys whatever the
-    // input's order and the jobs beside them, so theirs are put in it afterwards
-    // (launch_light_order), which pays where X has at least twice as many nonzeros
-    // for every free index as a light row may have products: few rows are light
-    // then, and all of them together have at most nx / 2 runs to sort.
-    bool by_free = con_tab;
-    uint64_t free_rows = 0;  // free indices of the jobs that may have light rows
+    // With the table the match does not care for the order of a row's nonzeros, so X
+    // is sorted by its free bits alone where that saves a radix pass (at the size
+    // above 4 -> 1 passes of 122 us).  Light rows add in the order of their contract
+    // keys whatever the input's order and the jobs beside them, so the planning puts
+    // their runs in it (k_matched_runs), which costs by the runs of a row: 8e6 X
+    // nonzeros in rows of 2 / 8 / 32 / 64 / 1000 runs of one product take 2.39 / 1.51 /
+    // 1.42 / 1.55 / 1.61 ms so and 2.57 / 1.57 / 1.37 / 1.36 / 1.39 sorted by all bits.
+    // So not where X has from 16 nonzeros for every free index up to twice what a
+    // light row may have products (past that few rows are light), nor for small
+    // inputs, where a launch more costs what the passes do.
+    const auto passes = [](int bits) { return (bits + 7) / 8; };
+    bool by_free = con_tab && nx >= kFreeSortNnz && passes(kbx + jb - min_ncb) < passes(kbx + jb);
+    bool any_light = false;
     for (Job *q : G) {
-        const int fb = q->LX.nfbits;
-        by_free &= !q->light_max || (fb < 32 && q->tx->nnz >= (2 * q->light_max) << fb);
-        if (q->light_max && fb < 32) free_rows += 1ull << fb;
+        const uint64_t a = q->LX.nfbits < 64 ? q->tx->nnz >> q->LX.nfbits : 0;
+        by_free &= a < 16 || a >= 2 * q->light_max;
+        any_light |= q->light_max != 0;
     }
     // relabeled jobs with 64-bit output keys
     bool any_wide = false;
@@ -806,7 +811,11 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         ra.lrun = lrun;
         ra.lrow = lrow;
         ra.loff = loff;
-        DBuf<uint32_t> row_mx;
+        DBuf<uint32_t> row_mx, longs;
+        if (by_free && any_light) {
+            longs.reset(A, nx / kOrderScan + 1, s);
+            ra.longs = longs;
+        }
         if (keep_bm) {
             row_mx.reset(A, nx, s);
             ra.row_rb = row_rb;
@@ -830,7 +839,7 @@ void run_group(gsparc_ctx *ctx, std::vector<Job *> &G, uint64_t max_chunk_nnz, i
         mark(3);
         launch_light_units(nx, light_bin, ra, cnts, scan_state(flags_x + 2 * zf_x), s);
         launch_matched_runs(nx, pos, cnt, rank, ra, cnts, plan_err, s);
-        if (by_free) launch_light_order(free_rows, pos, cnt, ra, cnts, plan_err, ctx->sm_count, s);
+        if (longs.get()) launch_light_order(nx, pos, cnt, ra, cnts, plan_err, ctx->sm_count, s);
         if (keep_bm)
             launch_heavy_bitmaps(nx, ra, bm_w_all, bm_w_dense, bm_off_all, bm_off_dense, cnts,
                                  scan_state(flags_x + 3 * zf_x), s);

@@ -409,6 +409,8 @@ __global__ void __launch_bounds__(kScanThreads)
             r.row_xi[row] = l;
             r.lpre[l] = x[2];
             r.lk0[l] = (uint32_t)x[4];
+            if (r.longs && rn[q] > kOrderScan)
+                r.longs[atomicAdd((unsigned long long *)&cnts[kCntLong], 1ull)] = l;
             x[1] += 1;
             x[2] += pr[q];
             x[4] += rn[q];
@@ -467,6 +469,13 @@ __global__ void __launch_bounds__(kScanThreads)
 // rank, so a run's first and last entries bound it); a warp whose nonzeros are
 // of one row (long rows) folds them first.  With a warp per row, 200 rows of
 // 5e4 runs took 1155 us (200 warps at work); now 146.
+//
+// Where X is sorted by its free bits alone, a light row's runs are put in the
+// order of their contract keys (the order of their first Y entries), equal keys
+// in input order, as a sort by all bits leaves them.  So a light row's sums
+// depend neither on the order of the input nor on the jobs beside it.  Up to
+// kOrderScan runs: a thread counts the runs before its own (loads that its
+// row's other threads make too); more: k_light_order.
 __global__ void k_matched_runs(const uint32_t *__restrict__ pos, const uint32_t *__restrict__ cnt,
                                const uint32_t *__restrict__ yrank, RowArrays r, const uint64_t *__restrict__ cnts,
                                const unsigned int *__restrict__ err) {
@@ -480,11 +489,27 @@ __global__ void k_matched_runs(const uint32_t *__restrict__ pos, const uint32_t 
         const uint32_t row = r.mrow[k < n ? k : n - 1];
         const uint8_t cl = k < n ? r.row_class[row] : kRowNone;
         if (cl == kRowLight) {
-            const uint32_t i = r.mrun[k], l = r.row_xi[row];
-            const uint32_t at = r.lk0[l] + (uint32_t)k - r.row_k0[row];
+            const uint32_t i = r.mrun[k], l = r.row_xi[row], k0r = r.row_k0[row], m = r.row_k0[row + 1] - k0r;
+            uint32_t at = (uint32_t)k - k0r;
+            uint64_t off = r.xprefix[i] - r.xprefix[r.row_start[row]];
+            if (r.longs && m <= kOrderScan) {
+                const uint32_t p = pos[i];
+                uint32_t n = 0;  // a light row has at most 2048 products
+                at = 0;
+#pragma unroll 4
+                for (uint32_t t = 0; t < m; ++t) {
+                    const uint32_t j = r.mrun[k0r + t], q = pos[j], c = cnt[j];
+                    if (q < p || (q == p && j < i)) {
+                        ++at;
+                        n += c;
+                    }
+                }
+                off = n;
+            }
+            at += r.lk0[l];
             r.lrun[at] = i;
             r.lrow[at] = l;
-            r.loff[at] = r.lpre[l] + r.xprefix[i] - r.xprefix[r.row_start[row]];
+            r.loff[at] = r.lpre[l] + off;
         }
         if (!row_rb) continue;  // the same in every thread
         const bool heavy = cl == kRowHeavy;
@@ -509,11 +534,8 @@ __global__ void k_matched_runs(const uint32_t *__restrict__ pos, const uint32_t 
     }
 }
 
-// Where X is sorted by its free bits alone, a CTA a light row: its runs in the
-// order of their contract keys (the order of their first Y entries), equal keys
-// in input order, as the sort by all bits leaves them.  So a light row's sums
-// depend neither on the order of the input nor on the jobs beside it.  Rows are
-// long there (batch.cu, by_free), so few are light: with none, 3 us.
+// The same order for the light rows of more than kOrderScan runs, a CTA a row: a
+// bitonic sort on chip (these rows are few; with none, 3 us).
 constexpr int kOrderRuns = 2048;  // a light row has no more products
 static_assert(kOrderRuns >= kLightCap / 2, "the largest light_row_max");
 __global__ void __launch_bounds__(kThreads)
@@ -523,9 +545,9 @@ __global__ void __launch_bounds__(kThreads)
     __shared__ uint64_t key[kOrderRuns];  // first Y entry, X nonzero
     __shared__ uint32_t s_tmp[33];
     if (*err & kScanErr) return;
-    const uint32_t n = (uint32_t)cnts[kCntLight], tid = threadIdx.x;
-    for (uint32_t l = blockIdx.x; l < n; l += gridDim.x) {
-        const uint32_t a = r.lk0[l], m = min(r.lk0[l + 1] - a, (uint32_t)kOrderRuns);
+    const uint32_t n = (uint32_t)cnts[kCntLong], tid = threadIdx.x;
+    for (uint32_t w = blockIdx.x; w < n; w += gridDim.x) {
+        const uint32_t l = r.longs[w], a = r.lk0[l], m = min(r.lk0[l + 1] - a, (uint32_t)kOrderRuns);
         uint32_t padded = 1;
         while (padded < m) padded <<= 1;
         __syncthreads();  // the row before this one has left `key`
@@ -706,10 +728,11 @@ void launch_matched_runs(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, 
     launched();
 }
 
-void launch_light_order(uint64_t rows, const uint32_t *pos, const uint32_t *cnt, const RowArrays &r,
+void launch_light_order(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, const RowArrays &r,
                         const uint64_t *cnts, const unsigned int *err, int sm_count, cudaStream_t s) {
-    if (rows == 0) return;
-    k_light_order<<<(unsigned)std::min<uint64_t>(rows, 8ull * sm_count), kThreads, 0, s>>>(pos, cnt, r, cnts, err);
+    if (nx <= kOrderScan) return;
+    k_light_order<<<(unsigned)std::min<uint64_t>(nx / kOrderScan + 1, 8ull * sm_count), kThreads, 0, s>>>(pos, cnt, r,
+                                                                                                       cnts, err);
     launched();
 }
 

@@ -34,7 +34,8 @@ enum {
     kCntProducts = 16,
     kCntErr = 17,        // error bits of the planning kernels and the radix sort (low word)
     kCntLightRuns = 18,  // runs of the light rows
-    kCnts = 19
+    kCntLong = 19,       // light rows of more than kOrderScan runs
+    kCnts = 20
 };
 
 constexpr uint8_t kRowNone = 0, kRowLight = 1, kRowStream = 2, kRowHeavy = 3, kRowNarrow = 4;  // narrow: heavy, over few columns
@@ -55,6 +56,8 @@ void launch_col_table(const uint32_t *bits, uint64_t nwords, const BPrep *jobs, 
 void launch_y_ranks(const uint64_t *ykeys, uint64_t ny, int kby, const BPrep *jobs, int g, const uint32_t *bits,
                     const uint32_t *wpre, const uint64_t *cnts, uint32_t *rank, BatchJob *acc,
                     const unsigned int *ydup, const unsigned int *err, cudaStream_t s);
+
+constexpr uint32_t kOrderScan = 64;
 
 struct RowArrays {
     uint64_t *xprefix;   // [nx + 1] matched products before every X nonzero
@@ -77,6 +80,9 @@ struct RowArrays {
     uint32_t *lrun;      // [light runs] their X nonzeros, light row after light row
     uint32_t *lrow;      // [light runs] their light rows (indices into L)
     uint64_t *loff;      // [light runs] products of the light rows' runs before each one
+    // X sorted by its free bits alone (null: by all bits): [nx / kOrderScan + 1]
+    // the light rows (indices into L) of more than kOrderScan runs, in any order
+    uint32_t *longs;
     uint32_t *row_rb, *row_mx;  // heavy rows: all ones and 0 (null: not wanted)
 };
 // Match of every X nonzero -> prefix sums, matched list and rows.
@@ -101,14 +107,13 @@ void launch_row_classes(uint64_t nx, const BPrep *jobs, const BatchJob *acc, con
 // Light units: consecutive light rows of fewer than bin + light_max products.
 void launch_light_units(uint64_t nx, uint64_t bin, const RowArrays &r, uint64_t *cnts, const ScanState &st,
                         cudaStream_t s);
-// The light rows' runs (lrun, lrow, loff) and, with row_rb and row_mx, the rank
-// span of every heavy row.
+// The light rows' runs (lrun, lrow, loff; with `longs`, those of rows of up to
+// kOrderScan runs in the order of their contract keys) and, with row_rb and
+// row_mx, the rank span of every heavy row.
 void launch_matched_runs(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, const uint32_t *yrank,
                          const RowArrays &r, const uint64_t *cnts, const unsigned int *err, cudaStream_t s);
-// Where X is sorted by its free bits alone: the light rows' runs (lrun, loff) in
-// the order of their contract keys, equal ones in input order.  `rows`: the most
-// light rows there can be.
-void launch_light_order(uint64_t rows, const uint32_t *pos, const uint32_t *cnt, const RowArrays &r,
+// The runs (lrun, loff) of the rows in `longs` in the order of their contract keys.
+void launch_light_order(uint64_t nx, const uint32_t *pos, const uint32_t *cnt, const RowArrays &r,
                         const uint64_t *cnts, const unsigned int *err, int sm_count, cudaStream_t s);
 // Kept bitmaps: of every heavy row the words with all / only dense
 // rows kept (w_*, by row), their word offsets (off_*, by row) and totals.

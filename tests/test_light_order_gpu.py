@@ -1,7 +1,7 @@
 """The order in which a light row adds its products: that of the contract keys,
 whatever the order of the input, the jobs beside it in a batch, and the bits
-that X is sorted by (long rows of mostly unmatched nonzeros are sorted by their
-free bits alone).  The sums cancel to a 1e-9th of their terms, so that another
+that X is sorted by (from 4,096 nonzeros on by their free bits alone; the rows
+are padded with unmatched nonzeros to both sides of that).  The sums cancel to a 1e-9th of their terms, so that another
 order shows in the last bits; the values are compared bit for bit with the same
 compensated sums in float32 on the CPU."""
 import numpy as np
@@ -11,7 +11,7 @@ import gsparc_b200 as gb
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(45, 6), (33, 31), (3, 300), (1000, 1), (1024, 1)]  # contract keys, columns: products of a row
+SHAPES = [(45, 6), (33, 31), (3, 300), (64, 3), (65, 3), (127, 8), (128, 8), (1000, 1), (1024, 1)]  # contract keys, columns: products of a row
 
 
 @pytest.fixture(scope="module")
@@ -53,7 +53,7 @@ def _shuffled(X, seed):
     return gb.CooTensor(X.dims, X.idx[:, p].copy(), X.val[p].copy())
 
 
-@pytest.mark.parametrize("unmatched", [0, 5000])
+@pytest.mark.parametrize("unmatched", [0, 5000, 12000])
 @pytest.mark.parametrize("keys,cols", SHAPES)
 def test_input_order(ctx, keys, cols, unmatched):
     X, Y, want = _job(keys, cols, 1 << 14, 2, unmatched, keys)
@@ -66,7 +66,7 @@ def test_input_order(ctx, keys, cols, unmatched):
 @pytest.mark.parametrize("keys,cols", SHAPES)
 def test_company(ctx, keys, cols):
     # contract keys of 12, 14, 17 and 6 bits, short and long rows
-    jobs = [_job(keys, cols, 1 << 12, 40, 0, 1), _job(keys, cols, 1 << 14, 2, 5000, 2), _job(keys, cols, 1 << 17, 7, 0, 3),
+    jobs = [_job(keys, cols, 1 << 12, 40, 0, 1), _job(keys, cols, 1 << 14, 2, 12000, 2), _job(keys, cols, 1 << 17, 7, 0, 3),
             _job(min(keys, 60), cols, 1 << 6, 9, 0, 4)]
     for pick in ([0, 1, 2, 3], [1, 1], [3, 1], [2, 0]):
         dev = [(ctx.upload(_shuffled(jobs[k][0], k)), ctx.upload(jobs[k][1])) for k in pick]
