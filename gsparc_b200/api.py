@@ -676,7 +676,8 @@ def sptc_host(ctx: Context, X: CooTensor, Y: CooTensor, cx: Sequence[int], cy: S
     (gsparc_sptc_host): X is cut into output-row parts and Y into
     output-column parts (of at most max_part_nnz_* nonzeros, or sized from the
     budget), every pair is contracted, Z arrives in key order.  sink: "host"
-    (Z returned as numpy arrays) or "discard"."""
+    (Z returned as numpy arrays, copied in pieces of at most ``staging``
+    nonzeros, and of STAGING_NNZ at most) or "discard"."""
     if len(cx) != len(cy):
         raise ValueError("cx and cy must have the same length")
     c1 = np.asarray(cx, np.int32)
@@ -839,7 +840,8 @@ def sptc_batch(ctx: Context, jobs, sink: str = "host", max_chunk_nnz: int = 0, s
 
     jobs: sequence of ``(X, Y, cx, cy)`` or ``(X, Y, cx, cy, accum)`` with
     resident DeviceTensors.  sink: "host" (every job's Z copied into numpy
-    arrays through one shared staging buffer of ``staging`` entries),
+    arrays through one shared staging buffer of ``staging`` entries, STAGING_NNZ
+    at most),
     "discard", or "device" (``on_chunk(job, keys_ptr, vals_ptr, n, first)``
     with device pointers).  Returns ``(results, batch_stats)``; a failed job's
     result has ``keys is None`` and its status in ``stats["status"]``.
@@ -965,7 +967,9 @@ class Server:
 
     def submit(self, X: ServerTensor, Y: ServerTensor, cx: Sequence[int], cy: Sequence[int],
                dense_accumulator: int = ACCUM_AUTO, sink: str = "host", staging: int = 1 << 20) -> int:
-        """Queue Z = X x_{cx,cy} Y; sink "host" (Z returned by wait) or "discard"."""
+        """Queue Z = X x_{cx,cy} Y; sink "host" (Z returned by wait, copied in
+        pieces of at most ``staging`` nonzeros, and of STAGING_NNZ at most) or
+        "discard"."""
         if len(cx) != len(cy):
             raise ValueError("cx and cy must have the same length")
         c1 = np.asarray(cx, np.int32)

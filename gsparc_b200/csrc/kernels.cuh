@@ -176,9 +176,10 @@ void launch_heavy(const AccArgs &a, bool numeric, int grid, cudaStream_t s);
 constexpr uint64_t kKeepBitsPerProduct = 32;
 constexpr uint64_t kKeepBitsMax = 512;
 // Narrow rows (narrow.cu): heavy rows of jobs with at most kNarrowCols distinct
-// columns and at least kNarrowProducts products a column.  8 warps' pairs of
-// 1024 columns are 64 KB, three CTAs an SM; the products a column pay for
-// adding the warps' pairs up and for the marks (32 words a row).
+// columns and at least kNarrowProducts products a column.  8 warps' pairs and
+// tags of 1024 columns are 72 KB (with the staged runs 76 KB): two CTAs an SM,
+// three from 1020 columns down; the products a column pay for adding the warps'
+// pairs up and for the marks (32 words a row).
 constexpr int kNarrowCols = 1024;
 constexpr uint64_t kNarrowProducts = 16;
 constexpr uint64_t kNarrowSlice = 16384;  // products of a unit at least (2048 a warp)

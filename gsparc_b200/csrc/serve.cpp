@@ -61,7 +61,9 @@ struct Lane {
 // Peak working memory of one job's linearise / sort / run table / match /
 // row planning, per operand nonzero, with headroom for CUB temporaries (the
 // buffers run_group holds at its high-water mark: ~160 B per X nonzero and
-// ~60 B per Y nonzero).
+// ~60 B per Y nonzero).  The presence bits and the run lookup table come on top:
+// run_group takes them out of the output window the batch was admitted with,
+// each within a quarter of what this estimate leaves of its budget.
 uint64_t job_estimate(const gsparc_job &J) {
     return 192ull * J.x->nnz + 96ull * J.y->nnz + (8ull << 20);
 }
